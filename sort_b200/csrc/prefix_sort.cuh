@@ -331,8 +331,15 @@ __global__ void __launch_bounds__(kSortThreads) k_digit_scatter(const K* __restr
 inline int sort_tiles(int64_t n) { return (int)((n + kSortTile - 1) / kSortTile); }
 // Words of count scratch a sort of n keys needs (digit-major counts).
 inline size_t sort_count_words(int64_t n) { return (size_t)kDigits * (size_t)sort_tiles(n); }
-// Words of scan scratch a sort of n keys needs.
-inline size_t sort_scan_words(int64_t n) { return scan_scratch_words(sort_count_words(n)); }
+// A sort pass scans its counts in two levels of kScanTile tiles while one
+// block can scan the tiles' totals, by scan_exclusive beyond.
+inline size_t sort_scan_tiles(int64_t n) { return (sort_count_words(n) + kScanTile - 1) / kScanTile; }
+inline bool sort_two_level(int64_t n) { return sort_scan_tiles(n) <= 1024; }
+// Words of scan scratch a sort of n keys needs: the two-level scan keeps one
+// total per kScanTile tile, more words than scan_exclusive's coarser tiles.
+inline size_t sort_scan_words(int64_t n) {
+    return sort_two_level(n) ? sort_scan_tiles(n) : scan_scratch_words(sort_count_words(n));
+}
 
 // Sorts n (key, value) pairs by key bits [begin_bit, end_bit), stably, in
 // passes of kDigitBits (the last may be narrower; the digit mask reads any
@@ -346,7 +353,7 @@ cudaError_t sort_pairs(K* keys[2], int32_t* vals[2], int64_t n, int begin_bit, i
     if (n <= 0) return cudaSuccess;
     const int tiles = sort_tiles(n);
     const size_t counts = sort_count_words(n);
-    const size_t scan_tiles = (counts + kScanTile - 1) / kScanTile;
+    const size_t scan_tiles = sort_scan_tiles(n);
     cudaError_t e = cudaSuccess;
     int cur = 0;
     for (int shift = begin_bit; shift < end_bit && e == cudaSuccess; shift += kDigitBits) {
@@ -355,7 +362,7 @@ cudaError_t sort_pairs(K* keys[2], int32_t* vals[2], int64_t n, int begin_bit, i
             if ((e = cudaGetLastError()) != cudaSuccess) break;
         }
         const uint32_t* tile_start = nullptr;
-        if (scan_tiles <= 1024) {  // two levels; the scatter adds the tile's start itself
+        if (sort_two_level(n)) {  // two levels; the scatter adds the tile's start itself
             k_scan_tiles<<<(unsigned)scan_tiles, 1024, 0, s>>>(count, count, counts, scan);
             k_scan_tile_sums<<<1, 1024, 0, s>>>(scan, (int)scan_tiles);
             tile_start = scan;
