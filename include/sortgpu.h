@@ -154,24 +154,25 @@ typedef struct {
     int32_t build_launches;  /* GPU builders: their split / collapse kernels launched (prefix sums and sorts not counted) */
 } sg_scene_info;
 
-/* Traversal launch schedule (results never depend on it). */
+/* Traversal launch schedule: the order in which a batch's rays are taken
+ * (results never depend on it). Every schedule runs the warp-cooperative
+ * kernel, in which idle lanes take the batch's next rays. */
 typedef enum {
-    SG_SCHEDULE_THREAD_PER_RAY = 0, /* one ray per thread for the whole launch */
-    SG_SCHEDULE_PERSISTENT = 1,     /* persistent warps; a finished lane takes the batch's next ray */
-    SG_SCHEDULE_WHILE_WHILE = 2,    /* each warp alternates an interior phase and a leaf phase */
-    SG_SCHEDULE_SPECULATIVE = 3,    /* while-while; lanes keep descending past their first leaf */
-    SG_SCHEDULE_SORTED = 4,         /* one ray per thread, threads given rays in the order of a 30-bit key
-                                       (direction octant, origin cell, coarse direction) so that a warp's
-                                       rays take similar paths; batches of 65,536 rays or more; scratch
-                                       (16 B per ray) from a stream-ordered pool */
+    SG_SCHEDULE_THREAD_PER_RAY = 0, /* batch order */
+    SG_SCHEDULE_PERSISTENT = 1,     /* batch order; new rays are taken at refill_threshold idle lanes */
+    SG_SCHEDULE_WHILE_WHILE = 2,    /* as THREAD_PER_RAY */
+    SG_SCHEDULE_SPECULATIVE = 3,    /* as THREAD_PER_RAY */
+    SG_SCHEDULE_SORTED = 4,         /* in the order of a 30-bit key (direction octant, origin cell, coarse
+                                       direction) so that concurrent warps read the same nodes; batches of
+                                       65,536 rays or more; scratch (16 B per ray) from a stream-ordered
+                                       pool */
     SG_SCHEDULE_AUTO = 5            /* a new scene's default: SORTED for closest-hit batches of 2M rays or
-                                       more (measured faster on 4M incoherent rays, slower on 1M coherent
-                                       primary rays), THREAD_PER_RAY otherwise */
+                                       more, THREAD_PER_RAY otherwise */
 } sg_schedule;
 
 typedef struct {
     int32_t schedule;          /* sg_schedule */
-    int32_t refill_threshold;  /* idle lanes (1..32) that make a persistent warp fetch new rays */
+    int32_t refill_threshold;  /* PERSISTENT: idle lanes (1..32) at which a warp takes new rays */
 } sg_trace_tuning;
 
 typedef struct sg_scene sg_scene;

@@ -48,7 +48,10 @@ __global__ void k_generate(Cam cam, int width, int height, int p0, int n, uint2 
     q.slot[p] = p;
     thr[p] = thr[cap + p] = thr[2 * cap + p] = 1.0f;          // throughput
     thr[3 * cap + p] = thr[4 * cap + p] = thr[5 * cap + p] = 0.0f;  // radiance of this sample
-    if (p == 0) *count = n;
+    if (p == 0) {
+        count[kCurrent] = n;
+        count[kExtendTaken] = 0;
+    }
 }
 
 __global__ void k_shade(PtDev sc, uint2 key, int p0, uint32_t sample, int bounce, int max_depth, Queue in, int cap,
@@ -360,7 +363,8 @@ cudaError_t pt_wave(const PtDev& dev, const TraceLaunch& base_in, const DevTree&
         Lc.any = false;
         Lc.prim = w.hit_prim;
         Lc.t = w.hit_t;
-        Lc.n_dev = &counters[0];
+        Lc.n_dev = &counters[kCurrent];
+        Lc.counter = reinterpret_cast<unsigned*>(&counters[kExtendTaken]);
         return launch_trace_fp32(Lc, tree, r, (int64_t)cap, s);
     };
     // Shadow rays, their results and the path radiance of bounce `cur` on
@@ -371,40 +375,41 @@ cudaError_t pt_wave(const PtDev& dev, const TraceLaunch& base_in, const DevTree&
         TraceLaunch La = base;
         La.any = true;
         La.occ = w.occ;
-        La.n_dev = &counters[2];
+        La.n_dev = &counters[kShadow];
+        La.counter = reinterpret_cast<unsigned*>(&counters[kShadowTaken]);
         cudaError_t r = launch_trace_fp32(La, tree, sr, (int64_t)scap, t);
         if (r != cudaSuccess) return r;
-        k_resolve<<<(scap + threads - 1) / threads, threads, 0, t>>>(sq, scap, &counters[2], w.occ, w.vis, cap);
+        k_resolve<<<(scap + threads - 1) / threads, threads, 0, t>>>(sq, scap, &counters[kShadow], w.occ, w.vis, cap);
         k_accumulate<<<blocks, threads, 0, t>>>(*q, shaded, w.vis, w.thr, cap);
-        k_count_rays<<<1, 32, 0, t>>>(shaded, &counters[2], w.totals);
+        k_count_rays<<<1, 32, 0, t>>>(shaded, &counters[kShadow], w.totals);
         return cudaGetLastError();
     };
     k_generate<<<blocks, threads, 0, s>>>(cam, width, height, p0, n, key, (uint32_t)sample, *cur, cap, w.thr,
-                                          &counters[0]);
+                                          counters);
     if ((e = closest(cur)) != cudaSuccess) return e;
     for (int bounce = 0; bounce < max_depth; ++bounce) {
-        if ((e = cudaMemsetAsync(&counters[1], 0, 2 * sizeof(int), s)) != cudaSuccess) return e;
+        if ((e = cudaMemsetAsync(&counters[kNext], 0, (kShadowTaken - kNext + 1) * sizeof(int), s)) != cudaSuccess) return e;
         k_shade<<<blocks, threads, 0, s>>>(dev, key, p0, (uint32_t)sample, bounce, max_depth, *cur, cap,
-                                           &counters[0], w.hit_prim, w.hit_t, *nxt, &counters[1], sq, scap,
-                                           &counters[2], w.thr, w.vis);
+                                           &counters[kCurrent], w.hit_prim, w.hit_t, *nxt, &counters[kNext], sq, scap,
+                                           &counters[kShadow], w.thr, w.vis);
         const bool more = bounce + 1 < max_depth;
         if (!w.side) {
-            if ((e = shadows(cur, &counters[0], s)) != cudaSuccess) return e;
+            if ((e = shadows(cur, &counters[kCurrent], s)) != cudaSuccess) return e;
         } else {
             // The shadow rays of this bounce go to the side stream and run
             // beside the next bounce's extension rays; the next shading (which
             // reuses the shadow queue, the path state and the counters) waits
             // for them.
-            if ((e = cudaMemcpyAsync(&counters[3], &counters[0], sizeof(int), cudaMemcpyDeviceToDevice, s)) !=
+            if ((e = cudaMemcpyAsync(&counters[kShaded], &counters[kCurrent], sizeof(int), cudaMemcpyDeviceToDevice, s)) !=
                     cudaSuccess ||
                 (e = cudaEventRecord(w.shaded, s)) != cudaSuccess ||
                 (e = cudaStreamWaitEvent(w.side, w.shaded, 0)) != cudaSuccess ||
-                (e = shadows(cur, &counters[3], w.side)) != cudaSuccess ||
+                (e = shadows(cur, &counters[kShaded], w.side)) != cudaSuccess ||
                 (e = cudaEventRecord(w.shadowed, w.side)) != cudaSuccess)
                 return e;
         }
         // the next queue becomes the current one
-        if ((e = cudaMemcpyAsync(&counters[0], &counters[1], sizeof(int), cudaMemcpyDeviceToDevice, s)) !=
+        if ((e = cudaMemcpyAsync(&counters[kCurrent], &counters[kNext], sizeof(int), cudaMemcpyDeviceToDevice, s)) !=
             cudaSuccess)
             return e;
         Queue* t = cur;
@@ -456,13 +461,13 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
 
     // Buffers, kInFlight times (samples in flight): two extension queues (rays +
     // slots), hits, one shadow queue of 2 entries per path (rays + slots +
-    // contributions), occlusion flags, throughput, shadow results, 4
+    // contributions), occlusion flags, throughput, shadow results, the queue
     // counters; then the shared ray totals.
     const size_t cap = (size_t)P, scap = 2 * (size_t)P;
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t qbytes = align(cap * 8 * 4) + align(cap * 4);
     const size_t set = 2 * qbytes + align(cap * 4) * 2 + align(scap * 8 * 4) + align(scap * 4) +
-                       align(scap * 3 * 4) + align(scap) + align(cap * 6 * 4) + align(cap * 6 * 4) + align(16);
+                       align(scap * 3 * 4) + align(scap) + align(cap * 6 * 4) + align(cap * 6 * 4) + align(sg::kWaveCounters * 4);
     const size_t need = sg::kInFlight * set + align(16);
     if (ps->buf_bytes < need) {
         if (ps->d_buf) cudaFree(ps->d_buf);
@@ -501,7 +506,7 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
         w[k].occ = (uint8_t*)take(scap);
         w[k].thr = (float*)take(cap * 24);  // throughput and radiance per path
         w[k].vis = (float*)take(cap * 24);  // two shadow results per path
-        w[k].counters = (int*)take(16);     // current, next, shadow queue; the shaded queue's length
+        w[k].counters = (int*)take(sg::kWaveCounters * 4);
         w[k].cap = (int)cap;
         w[k].side = ps->side[k];
         w[k].shaded = ps->shaded[k];

@@ -20,9 +20,13 @@ constexpr int kInFlight = 2;
 // extension queues (8 floats per ray with stride cap, a path index per
 // entry), the hits (cap each), the shadow queue (stride 2 * cap, three
 // contribution planes) and its occlusion flags, per-path throughput and
-// radiance (6 * cap floats) and shadow results (6 * cap), four queue
-// counters (current, next, shadow, and the shaded queue's length for the side
-// stream) and two ray totals (extension, shadow).
+// radiance (6 * cap floats) and shadow results (6 * cap), the queue
+// counters (kWaveCounters) and two ray totals (extension, shadow).
+// Indices into PtWave::counters: queue lengths (the shaded queue's copy is for
+// the side stream) and the ray counters of the two traversals. kNext up to
+// kShadowTaken are zeroed together before each shading.
+enum { kCurrent = 0, kNext = 1, kShadow = 2, kExtendTaken = 3, kShadowTaken = 4, kShaded = 5, kWaveCounters = 6 };
+
 struct PtWave {
     float* qa_ray;
     int* qa_slot;
@@ -36,7 +40,7 @@ struct PtWave {
     uint8_t* occ;
     float* thr;
     float* vis;
-    int* counters;  // 4: current, next and shadow queue lengths, the shaded queue's length
+    int* counters;  // kWaveCounters, see the indices below
     unsigned long long* totals;
     int cap;
     // Optional: a second stream on which each bounce's shadow rays run beside

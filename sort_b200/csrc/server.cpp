@@ -768,7 +768,7 @@ sg_status sg_server_create(const sg_server_opts* opts, sg_server** out) {
         S->lanes.resize(kSoloLanes);
         const size_t cap = C, scap = 2 * C;
         const size_t parts[] = {cap * 32, cap * 4, cap * 32, cap * 4, cap * 4, cap * 4, scap * 32, scap * 4,
-                                scap * 12, scap, cap * 24, cap * 24, 16};
+                                scap * 12, scap, cap * 24, cap * 24, sg::kWaveCounters * 4};
         constexpr int kParts = int(sizeof(parts) / sizeof(parts[0]));
         size_t set = 0;
         for (size_t x : parts) set += align_up(x);

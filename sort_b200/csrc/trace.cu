@@ -15,18 +15,13 @@
 // With FP32 child boxes and the same rounding, hits, distances and barycentrics
 // are bit-identical to SORT's.
 //
-// GPU-side choices that leave that order intact:
-//   * the entry SORT would pop right after pushing a node's children (the
-//     nearest) stays in registers and is descended into directly;
-//   * leaf triangles are fetched two at a time (the triangle array carries one
-//     padding slot), so the second's loads overlap the first's test;
-//   * schedules: one ray per thread for the whole launch; persistent warps in
-//     which a lane whose ray finished takes the next ray of the batch, so warps
-//     stay full instead of idling on their slowest ray; while-while and its
-//     speculative form; and one ray per thread with the rays taken in the order
-//     of a coherence key (direction octant, origin cell, coarse direction), so
-//     a warp's rays visit similar nodes (fewer idle lanes), which the automatic
-//     default uses for large closest-hit batches.
+// The hot kernel is k_trace_walk over warp_walk.cuh: a ray per lane, leaves
+// tested by eight lanes each, idle lanes refilled. Counting launches
+// (sg_trace_stats) run Traversal, one ray per thread, whose node and triangle
+// visits are SORT's one by one. Schedules change the order in which rays are
+// taken, never a result: batch order, or the order of a coherence key (direction
+// octant, origin cell, coarse direction), which the automatic default uses for
+// large closest-hit batches so that concurrent warps read the same nodes.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -35,6 +30,7 @@
 #include "prefix_sort.cuh"
 #include "trace_kernels.h"
 #include "traversal.cuh"
+#include "warp_walk.cuh"
 
 namespace sg {
 
@@ -62,239 +58,133 @@ __device__ __forceinline__ void trace_one_ray(const DevTree& tr, const DevRays& 
     tv.finish(i, prim_out, t_out, u_out, v_out, occ_out, stats);
 }
 
-// Launch bounds: registers limit the occupancy of these kernels. Left alone,
-// the compiler gives the width-8 any-hit kernel 61 registers (8 blocks of 128
-// per SM); held to 9 blocks it fits 56 with 8 bytes spilled and runs 5.8%
-// faster on 4M shadow rays. The others already fit their bound (width 8
-// closest 56, width 4 closest 55, width 4 any-hit 48 at 10 blocks).
-template <int W, bool ANY, int STACK, bool STATS, bool Q8 = false>
-__global__ void __launch_bounds__(128, (W == 4 && ANY) ? 10 : 9) k_trace_fp32(DevTree tr, DevRays rays, int64_t n, int32_t* __restrict__ prim_out,
-                                                    float* __restrict__ t_out, float* __restrict__ u_out,
-                                                    float* __restrict__ v_out, uint8_t* __restrict__ occ_out,
-                                                    int* __restrict__ err, unsigned long long* __restrict__ stats,
-                                                    const int* __restrict__ n_dev,
-                                                    const int32_t* __restrict__ order = nullptr) {
-    trace_one_ray<W, ANY, STACK, STATS, Q8>(tr, rays, n, prim_out, t_out, u_out, v_out, occ_out, err, stats, n_dev,
-                                           order);
-}
-
-// One ray per thread with RayWalk, the hot path for FP32 and 8-bit nodes. With
-// n_dev set the batch is min(n, *n_dev); with `order` set, thread k traces ray
-// order[k]. Held to 9 blocks of 128 per SM (56 registers): left alone the
-// compiler takes 94 registers (every node and triangle load in flight at
-// once); 8 blocks ran at 994 Mrays/s, 9 at 1,031, and 10 (48 registers)
-// spills inside the traversal loop and fell to 968 (one triangle per
-// iteration) or to about 240 (two).
+// The counting launches' kernel.
 template <int W, bool ANY, int STACK, bool Q8>
-__global__ void __launch_bounds__(128, 9)
-    k_trace_walk(DevTree tr, DevRays rays, int64_t n, int32_t* __restrict__ prim_out, float* __restrict__ t_out,
-                 float* __restrict__ u_out, float* __restrict__ v_out, uint8_t* __restrict__ occ_out,
-                 int* __restrict__ err, const int* __restrict__ n_dev, const int32_t* __restrict__ order) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n_dev && k >= (int64_t)*n_dev) return;
-    if (k >= n) return;
-    const int64_t i = order ? (int64_t)__ldg(order + k) : k;
-    uint2 stk[STACK];
-    RayWalk<W, ANY, STACK, Q8> w;
-    if (w.start(tr, rays, i))
-        while (!w.step(tr, stk, err)) {
-        }
-    w.finish(tr, i, prim_out, t_out, u_out, v_out, occ_out);
+__global__ void __launch_bounds__(128, 9) k_trace_stats(DevTree tr, DevRays rays, int64_t n,
+                                                        int32_t* __restrict__ prim_out, float* __restrict__ t_out,
+                                                        float* __restrict__ u_out, float* __restrict__ v_out,
+                                                        uint8_t* __restrict__ occ_out, int* __restrict__ err,
+                                                        unsigned long long* __restrict__ stats,
+                                                        const int* __restrict__ n_dev) {
+    trace_one_ray<W, ANY, STACK, true, Q8>(tr, rays, n, prim_out, t_out, u_out, v_out, occ_out, err, stats, n_dev,
+                                           nullptr);
 }
 
-// The same for 8-bit nodes, held to 9 blocks of 128 per SM: the decode leaves
-// the compiler at 72-80 registers (7 blocks); at 56 it spills 64 bytes and is
-// still 4.6% faster on 4M incoherent rays (more warps hide the node loads).
-template <int W, bool ANY, int STACK, bool STATS>
-__global__ void __launch_bounds__(128, 9) k_trace_q8(DevTree tr, DevRays rays, int64_t n, int32_t* __restrict__ prim_out,
-                                                     float* __restrict__ t_out, float* __restrict__ u_out,
-                                                     float* __restrict__ v_out, uint8_t* __restrict__ occ_out,
-                                                     int* __restrict__ err, unsigned long long* __restrict__ stats,
-                                                     const int* __restrict__ n_dev,
-                                                     const int32_t* __restrict__ order = nullptr) {
-    trace_one_ray<W, ANY, STACK, STATS, true>(tr, rays, n, prim_out, t_out, u_out, v_out, occ_out, err, stats, n_dev,
-                                             order);
-}
+// Launch shape of k_trace_walk per tree form: blocks of 128 per SM (registers:
+// 72 at 7 blocks hold the width-8 FP32 walk without a spill, 64 at 8 blocks the
+// others) and the idle lanes at which a warp takes new rays. Measured, same
+// box, width 8: 7 blocks 2.54 / 2.10 ms on 4M diffuse / shadow rays (21M
+// triangles), 8 blocks (88 bytes spilled) 2.98 / 2.25, 9 blocks 2.96 / 2.40.
+// 8-bit nodes: 0.338 / 0.334 / 0.336 ms at 7 / 8 / 9 blocks on 700k rays.
+// Width 4, 1M camera rays: 0.207 / 0.207 / 0.201 ms at 7 / 8 / 9 blocks with a
+// refill at 10 idle lanes, 0.198 / 0.200 at 16 (4 idle lanes: 6% slower).
+template <int W, bool Q8>
+struct WalkShape {
+    static constexpr int kBlocks = W == 8 && !Q8 ? 7 : 8;
+    static constexpr int kRefill = W == 8 ? 10 : 16;
+};
 
-// Persistent warps: a lane whose ray finished takes the next ray in batch order
-// once at least `refill` lanes of its warp are idle; the warp's leader claims
-// those rays from a launch-wide counter, so the whole GPU still advances
-// through the batch in order (neighbouring rays share tree nodes in L1/L2).
-template <int W, bool ANY, int STACK, bool STATS>
-__global__ void __launch_bounds__(128) k_trace_fp32_persistent(DevTree tr, DevRays rays, int64_t n,
-                                                               unsigned long long* __restrict__ counter, int refill,
-                                                               int32_t* __restrict__ prim_out, float* __restrict__ t_out,
-                                                               float* __restrict__ u_out, float* __restrict__ v_out,
-                                                               uint8_t* __restrict__ occ_out, int* __restrict__ err,
-                                                               unsigned long long* __restrict__ stats) {
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    Traversal<W, ANY, STACK, STATS, false, true> tv;
-    uint2 stk_mem[STACK];
-    tv.stk = stk_mem;
-    bool alive = false;
-    bool drained = false;  // warp-uniform: the counter has passed n
-    int64_t ray = -1;
-    for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, !alive);
-        if (idle != 0 && !drained) {
-            unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(counter, (unsigned long long)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if ((int64_t)base >= n) drained = true;
-            if (!alive) {
-                const int64_t idx = (int64_t)base + __popc(idle & lt_mask);
-                if (idx < n) {
-                    ray = idx;
-                    alive = tv.start(tr, rays, idx);
-                    if (!alive) tv.finish(idx, prim_out, t_out, u_out, v_out, occ_out, stats);
-                }
-            }
-        }
-        const unsigned busy0 = __ballot_sync(0xffffffffu, alive);
-        if (busy0 == 0) {
-            if (drained) break;
-            continue;
-        }
-        // Traverse until enough lanes are idle to be worth refilling.
-        for (;;) {
-            if (alive && tv.step(tr, err)) {
-                tv.finish(ray, prim_out, t_out, u_out, v_out, occ_out, stats);
-                alive = false;
-            }
-            const unsigned busy = __ballot_sync(0xffffffffu, alive);
-            if (busy == 0) break;
-            if (!drained && 32 - __popc(busy) >= refill) break;
-        }
+// Rays of a launch as its warps take them: one span of `span` rays per warp, or,
+// with a counter, as many as the warp has idle lanes from the launch's counter,
+// so that the whole GPU advances through the batch in order (neighbouring rays
+// read the same nodes) and no warp ends much before the others.
+struct TraceJob {
+    const DevTree& tr;
+    const DevRays& rays;
+    const int32_t* order;
+    int32_t* prim_out;
+    float* t_out;
+    float* u_out;
+    float* v_out;
+    uint8_t* occ_out;
+    unsigned* counter;
+    int n, span, step;  // step: rays between a warp's spans
+    int next, end;
+
+    __device__ __forceinline__ const DevTree& tree() const { return tr; }
+    __device__ __forceinline__ bool more() {
+        if (next < end) return true;
+        if (counter || end >= n - (step - span)) return false;
+        next = end + (step - span);
+        end = n - next < span ? n : next + span;
+        return true;
     }
-}
+    __device__ __forceinline__ bool take(bool idle, unsigned mask, int lane, WalkShared* sh, RayState& r,
+                                         const DevTree&) {
+        if (counter) {
+            unsigned b = 0;
+            if (lane == 0) b = atomicAdd(counter, (unsigned)__popc(mask));
+            b = __shfl_sync(kFullWarp, b, 0);
+            next = b < (unsigned)n ? (int)b : n;
+        }
+        const int k = next + __popc(mask & ((1u << lane) - 1u));
+        const bool got = idle && k < end;
+        next += __popc(mask);
+        if (!got) return false;
+        const int i = order ? __ldg(order + k) : k;
+        sh->ray[lane] = (uint32_t)i;
+        r.o[0] = rays.ox[i];
+        r.o[1] = rays.oy[i];
+        r.o[2] = rays.oz[i];
+        r.d[0] = rays.dx[i];
+        r.d[1] = rays.dy[i];
+        r.d[2] = rays.dz[i];
+        r.tmin = rays.tmin[i];
+        r.tmax = rays.tmax[i];
+        return true;
+    }
+    __device__ __forceinline__ void put(bool fin, int lane, const WalkShared* sh) const {
+        if (!fin) return;
+        const uint32_t i = sh->ray[lane] & kWalkRayMask;
+        const int32_t prim = sh->prim[lane];
+        if (occ_out) {
+            occ_out[i] = prim >= 0 ? 1 : 0;
+            return;
+        }
+        prim_out[i] = prim;
+        t_out[i] = sh->t[lane];
+        if (u_out) u_out[i] = prim >= 0 ? sh->u[lane] : 0.0f;
+        if (v_out) v_out[i] = prim >= 0 ? sh->v[lane] : 0.0f;
+    }
+};
 
-// Persistent warps over RayWalk (the persistent schedule without counters): a
-// lane whose ray finished takes the next ray once at least `refill` lanes of
-// its warp are idle; the warp's leader claims those rays from a launch-wide
-// counter, in batch order or, with `order` set, in the order it lists.
+constexpr int kMaxWalkRays = 1 << 30;  // per launch: ray indices of 30 bits
+constexpr int kWalkSpan = 64;          // rays per warp of a large launch that has no counter
+static_assert(kMaxWalkRays - 1 <= (int)kWalkRayMask, "a ray's index fits its shared word");
+
+// Traces min(n, *n_dev) rays (n_dev may be null); with `order` set, the k-th ray
+// taken is ray order[k]. slots: warps the GPU holds at once. Up to 32 rays per
+// such warp each warp gets an equal share, so that a small batch spreads over
+// every SM (a ray's chain of dependent loads is what a small launch waits for);
+// beyond, warps take rays from `counter` (zero at launch) or by spans.
 template <int W, bool ANY, int STACK, bool Q8>
-__global__ void __launch_bounds__(128, 9)
-    k_trace_walk_persistent(DevTree tr, DevRays rays, int64_t n, unsigned long long* __restrict__ counter, int refill,
-                            const int32_t* __restrict__ order, int32_t* __restrict__ prim_out,
-                            float* __restrict__ t_out, float* __restrict__ u_out, float* __restrict__ v_out,
-                            uint8_t* __restrict__ occ_out, int* __restrict__ err) {
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    uint2 stk[STACK];
-    RayWalk<W, ANY, STACK, Q8> w;
-    bool alive = false;
-    bool drained = false;  // warp-uniform: the counter has passed n
-    int64_t ray = -1;
-    for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, !alive);
-        if (idle != 0 && !drained) {
-            unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(counter, (unsigned long long)__popc(idle));
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if ((int64_t)base >= n) drained = true;
-            if (!alive) {
-                const int64_t k = (int64_t)base + __popc(idle & lt_mask);
-                if (k < n) {
-                    ray = order ? (int64_t)__ldg(order + k) : k;
-                    alive = w.start(tr, rays, ray);
-                    if (!alive) w.finish(tr, ray, prim_out, t_out, u_out, v_out, occ_out);
-                }
-            }
-        }
-        const unsigned busy0 = __ballot_sync(0xffffffffu, alive);
-        if (busy0 == 0) {
-            if (drained) break;
-            continue;
-        }
-        for (;;) {  // traverse until enough lanes are idle to be worth refilling
-            if (alive && w.step(tr, stk, err)) {
-                w.finish(tr, ray, prim_out, t_out, u_out, v_out, occ_out);
-                alive = false;
-            }
-            const unsigned busy = __ballot_sync(0xffffffffu, alive);
-            if (busy == 0) break;
-            if (!drained && 32 - __popc(busy) >= refill) break;
-        }
+__global__ void __launch_bounds__(kWalkThreads, WalkShape<W, Q8>::kBlocks)
+    k_trace_walk(const __grid_constant__ DevTree tr, const __grid_constant__ DevRays rays, int n, int slots, int refill,
+                 int32_t* __restrict__ prim_out, float* __restrict__ t_out, float* __restrict__ u_out,
+                 float* __restrict__ v_out, uint8_t* __restrict__ occ_out, int* __restrict__ err,
+                 const int* __restrict__ n_dev, const int32_t* __restrict__ order, unsigned* __restrict__ counter) {
+    __shared__ WalkShared shared[kWalkWarps];
+    const int lane = threadIdx.x & 31, warp = (int)blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
+    if (n_dev) n = min(n, *n_dev);
+    int span = kWalkSpan;
+    if (n <= slots * 32) {
+        span = (n + slots - 1) / slots;
+        counter = nullptr;
     }
+    TraceJob job{tr, rays, order, prim_out, t_out, u_out, v_out, ANY ? occ_out : nullptr, counter, n, span, 0, 0, n};
+    if (!counter) {
+        const int64_t first = (int64_t)warp * span;
+        if (first >= n) return;
+        job.step = (int)gridDim.x * kWalkWarps * span;
+        job.next = (int)first;
+        job.end = n - job.next < span ? n : job.next + span;
+    }
+    walk_rays<W, ANY, STACK, Q8, false>(job, shared + (threadIdx.x >> 5), lane, refill, err);
 }
 
-// While-while traversal over RayWalk, one ray per thread: the warp alternates
-// an interior phase (each lane pops / descends until it holds an un-culled
-// leaf; with SPEC a lane that holds one keeps descending while others lack
-// one) and a leaf phase. Leaves are tested in SORT's order and culled with the
-// hit found so far, so results are SORT's: a speculative visit only sees
-// interior nodes SORT visits too, or that SORT culls -- and then every leaf
-// below is culled here as well, because a child's entry distance is never
-// below its parent's (each slab bound of a child lies inside the parent's, and
-// the rounded t = -o/d + b/d is monotonic in b). With `order` set, thread k
-// traces ray order[k]. Measured on 4,194,304 incoherent rays: 850 (plain) and
-// 902 (speculative) Mrays/s against 969 for one ray per thread, and 900 / 960
-// against 1,036 in sorted order: the phase bookkeeping costs more issue slots
-// than the split saves.
-template <int W, bool ANY, int STACK, bool SPEC>
-__global__ void __launch_bounds__(128, 9)
-    k_trace_walk_ww(DevTree tr, DevRays rays, int64_t n, const int32_t* __restrict__ order,
-                    int32_t* __restrict__ prim_out, float* __restrict__ t_out, float* __restrict__ u_out,
-                    float* __restrict__ v_out, uint8_t* __restrict__ occ_out, int* __restrict__ err) {
-    const int64_t k0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = k0 < n;
-    const int64_t k = valid ? k0 : n - 1;  // lanes past the batch end idle through the loop
-    const int64_t i = order ? (int64_t)__ldg(order + k) : k;
-    uint2 stk[STACK];
-    RayWalk<W, ANY, STACK, false> w;
-    const bool started = w.start(tr, rays, i);
-    bool have = valid && started;
-    bool pend = false;
-    int32_t lf = 0;
-    float lf_d = 0.0f;
-    while (__any_sync(0xffffffffu, have || pend)) {
-        for (;;) {
-            const bool needs = have && !pend;
-            const bool spec = SPEC && have && pend;
-            if (!__any_sync(0xffffffffu, needs)) break;
-            if (needs || spec) {
-                bool descend = false;
-                bool blocked = false;
-                if (!(w.best_t < w.cur_d)) {
-                    if (w.cur < 0) {
-                        if (w.cur == kEmpty) {
-                        } else if (!pend) {
-                            lf = w.cur;
-                            lf_d = w.cur_d;
-                            pend = true;
-                        } else {
-                            blocked = true;  // second leaf: wait for the leaf phase
-                        }
-                    } else if (w.si + W > STACK) {  // cannot happen when STACK >= depth*(W-1)+1
-                        atomicOr(err, 1);
-                        have = false;
-                        blocked = true;
-                    } else {
-                        descend = w.interior(tr, stk);
-                    }
-                }
-                if (!descend && !blocked) {
-                    if (w.si == 0) {
-                        have = false;
-                    } else {
-                        const uint2 e = stk[--w.si];
-                        w.cur = (int32_t)e.x;
-                        w.cur_d = __uint_as_float(e.y);
-                    }
-                }
-            }
-        }
-        if (pend) {
-            pend = false;
-            if (!(w.best_t < lf_d) && w.leaf(tr, lf)) have = false;  // any-hit: done
-        }
-    }
-    if (valid) w.finish(tr, i, prim_out, t_out, u_out, v_out, occ_out);
-}
-
-// Stream-ordered scratch for the sorted schedule: one pool per device that
-// keeps up to 1 GiB mapped between launches (NULL if it cannot be made).
+// Stream-ordered scratch of a launch (the sorted schedule's keys and order, the
+// ray counter): one pool per device that keeps up to 1 GiB mapped between
+// launches (NULL if it cannot be made).
 static cudaMemPool_t trace_scratch_pool(int device) {
     static std::mutex lock;
     static std::vector<cudaMemPool_t> pools;
@@ -313,6 +203,55 @@ static cudaMemPool_t trace_scratch_pool(int device) {
         pools[size_t(device)] = pool;
     }
     return pools[size_t(device)];
+}
+
+// Launches k_trace_walk over n rays, with the launch's counter or without one.
+template <int W, bool ANY, int STACK, bool Q8>
+static cudaError_t launch_walk(const TraceLaunch& L, const DevTree& tr, const DevRays& rays, int64_t n,
+                               const int32_t* order, unsigned* counter, cudaStream_t s) {
+    using Shape = WalkShape<W, Q8>;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const int slots = (sms < 1 ? 1 : sms) * Shape::kBlocks * kWalkWarps;
+    const int refill = L.tuning.schedule == kSchedulePersistent ? L.tuning.refill_threshold : Shape::kRefill;
+    // A large launch takes its rays from a counter: the caller's, or one from the
+    // scratch pool (not while the stream is captured: a graph may be replayed
+    // beside itself, and callers that asked for no scratch get none).
+    char* scratch = nullptr;
+    cudaMemPool_t pool = nullptr;
+    if (!counter && L.scratch && !L.n_dev && n > (int64_t)slots * 32) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
+            (void)cudaGetLastError();
+            cap = cudaStreamCaptureStatusActive;
+        }
+        if (cap == cudaStreamCaptureStatusNone && (pool = trace_scratch_pool(dev)) != nullptr) {
+            if ((e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), 256, pool, s)) != cudaSuccess) return e;
+            counter = reinterpret_cast<unsigned*>(scratch);
+        }
+    }
+    for (int64_t a = 0; a < n && e == cudaSuccess; a += kMaxWalkRays) {
+        const int m = (int)(n - a < kMaxWalkRays ? n - a : kMaxWalkRays);
+        int64_t warps = slots;
+        if (m <= slots * 32)
+            warps = m < slots ? m : slots;
+        else if (!counter && !L.n_dev)
+            warps = (m + kWalkSpan - 1) / kWalkSpan;
+        if (scratch && (e = cudaMemsetAsync(counter, 0, sizeof(unsigned), s)) != cudaSuccess) break;
+        const DevRays r{rays.ox + a, rays.oy + a, rays.oz + a,   rays.dx + a,
+                        rays.dy + a, rays.dz + a, rays.tmin + a, rays.tmax + a};
+        k_trace_walk<W, ANY, STACK, Q8><<<(unsigned)((warps + kWalkWarps - 1) / kWalkWarps), kWalkThreads, 0, s>>>(
+            tr, r, m, slots, refill, ANY ? nullptr : L.prim + a, ANY ? nullptr : L.t + a, L.u ? L.u + a : nullptr,
+            L.v ? L.v + a : nullptr, ANY ? L.occ + a : nullptr, L.err, L.n_dev, order, counter);
+        e = cudaGetLastError();
+    }
+    if (scratch) {
+        const cudaError_t f = cudaFreeAsync(scratch, s);
+        if (e == cudaSuccess) e = f;
+    }
+    return e;
 }
 
 // ---------------------------------------------------------------------------
@@ -368,7 +307,9 @@ __device__ __forceinline__ uint32_t spread7(uint32_t v) {  // bit b of v to bit 
 // counts of the first pass's digit (as k_digit_count).
 __global__ void __launch_bounds__(kSortThreads) k_sort_keys(DevRays rays, int64_t n, KeyGrid g, int shift, int tiles,
                                                             uint32_t* __restrict__ keys, int32_t* __restrict__ index,
-                                                            uint32_t* __restrict__ count) {
+                                                            uint32_t* __restrict__ count,
+                                                            unsigned* __restrict__ counter) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;  // the traversal's
     __shared__ uint32_t hist[kDigits];
     for (int d = threadIdx.x; d < kDigits; d += kSortThreads) hist[d] = 0;
     __syncthreads();
@@ -413,12 +354,13 @@ static cudaError_t launch_sorted(const TraceLaunch& L, const DevTree& tr, const 
     const size_t b_ray = up(size_t(n) * 4), b_count = up(psort::sort_count_words(n) * 4),
                  b_scan = up(psort::sort_scan_words(n) * 4);
     char* base = nullptr;
-    e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&base), 4 * b_ray + b_count + b_scan, pool, s);
+    e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&base), 4 * b_ray + b_count + b_scan + al, pool, s);
     if (e != cudaSuccess) return e;
     uint32_t* keys[2] = {reinterpret_cast<uint32_t*>(base), reinterpret_cast<uint32_t*>(base + b_ray)};
     int32_t* idx[2] = {reinterpret_cast<int32_t*>(base + 2 * b_ray), reinterpret_cast<int32_t*>(base + 3 * b_ray)};
     uint32_t* count = reinterpret_cast<uint32_t*>(base + 4 * b_ray);
     uint32_t* scan = reinterpret_cast<uint32_t*>(base + 4 * b_ray + b_count);
+    unsigned* counter = reinterpret_cast<unsigned*>(base + 4 * b_ray + b_count + b_scan);
     KeyGrid g;
     for (int a = 0; a < 3; ++a) {
         const float ext = tr.box_hi[a] - tr.box_lo[a];
@@ -426,15 +368,12 @@ static cudaError_t launch_sorted(const TraceLaunch& L, const DevTree& tr, const 
         g.scale[a] = ext > 0.0f ? 128.0f / ext : 0.0f;
     }
     const int first = kKeyBits - kSortBits;
-    k_sort_keys<<<tiles, kSortThreads, 0, s>>>(rays, n, g, first, tiles, keys[0], idx[0], count);
+    k_sort_keys<<<tiles, kSortThreads, 0, s>>>(rays, n, g, first, tiles, keys[0], idx[0], count,
+                                               counter);
     int cur = 0;
     if ((e = cudaGetLastError()) == cudaSuccess)
         e = psort::sort_pairs<uint32_t>(keys, idx, n, first, kKeyBits, count, scan, true, &cur, s);
-    if (e == cudaSuccess) {
-        k_trace_walk<W, ANY, STACK, Q8><<<(unsigned)((n + 127) / 128), 128, 0, s>>>(
-            tr, rays, n, L.prim, L.t, L.u, L.v, L.occ, L.err, nullptr, idx[cur]);
-        e = cudaGetLastError();
-    }
+    if (e == cudaSuccess) e = launch_walk<W, ANY, STACK, Q8>(L, tr, rays, n, idx[cur], counter, s);
     const cudaError_t f = cudaFreeAsync(base, s);
     return e != cudaSuccess ? e : f;
 }
@@ -442,81 +381,27 @@ static cudaError_t launch_sorted(const TraceLaunch& L, const DevTree& tr, const 
 template <int W, bool ANY, int STACK, bool STATS>
 static cudaError_t launch_stack(const TraceLaunch& L, const DevTree& tr, const DevRays& rays, int64_t n,
                                 cudaStream_t s) {
-    const int threads = 128;
-    // Batches large enough for reordering to pay (and within a 32-bit sort);
-    // the automatic choice sorts large closest-hit batches only (any-hit rays
-    // end early, and measured no faster sorted).
+    if (STATS) {
+        const unsigned blocks = (unsigned)((n + 127) / 128);
+        if (L.q8)
+            k_trace_stats<W, ANY, STACK, true><<<blocks, 128, 0, s>>>(tr, rays, n, L.prim, L.t, L.u, L.v, L.occ, L.err,
+                                                                      L.stats, L.n_dev);
+        else
+            k_trace_stats<W, ANY, STACK, false><<<blocks, 128, 0, s>>>(tr, rays, n, L.prim, L.t, L.u, L.v, L.occ, L.err,
+                                                                       L.stats, L.n_dev);
+        return cudaGetLastError();
+    }
+    // Batches large enough for reordering to pay; the automatic choice sorts
+    // large closest-hit batches only (any-hit rays end early, and measured no
+    // faster sorted).
     const bool sorted = L.tuning.schedule == kScheduleSorted ? n >= (int64_t(1) << 16)
                         : L.tuning.schedule == kScheduleAuto  ? !ANY && n >= (int64_t(1) << 21)
                                                               : false;
-    if (!STATS && !L.n_dev && sorted && n < (int64_t(1) << 31))
+    if (!L.n_dev && sorted && n <= kMaxWalkRays)
         return L.q8 ? launch_sorted<W, ANY, STACK, true>(L, tr, rays, n, s)
                     : launch_sorted<W, ANY, STACK, false>(L, tr, rays, n, s);
-    // Counting launches keep the one-entry-per-step loop, whose interior-node
-    // visits are exactly SORT's (speculation visits extra ones).
-    // 8-bit nodes are read by the one-ray-per-thread kernels.
-    if (L.q8) {
-        const int64_t blocks = (n + threads - 1) / threads;
-        if (STATS)
-            k_trace_q8<W, ANY, STACK, STATS><<<(unsigned)blocks, threads, 0, s>>>(
-                tr, rays, n, L.prim, L.t, L.u, L.v, L.occ, L.err, L.stats, L.n_dev);
-        else
-            k_trace_walk<W, ANY, STACK, true><<<(unsigned)blocks, threads, 0, s>>>(
-                tr, rays, n, L.prim, L.t, L.u, L.v, L.occ, L.err, L.n_dev, nullptr);
-        return cudaGetLastError();
-    }
-    // A device-side batch size is only read by the one-ray-per-thread kernel.
-    if (!STATS && !L.n_dev &&
-        (L.tuning.schedule == kScheduleWhileWhile || L.tuning.schedule == kScheduleSpeculative)) {
-        const int64_t blocks = (n + threads - 1) / threads;
-        if (L.tuning.schedule == kScheduleSpeculative)
-            k_trace_walk_ww<W, ANY, STACK, true><<<(unsigned)blocks, threads, 0, s>>>(tr, rays, n, nullptr, L.prim,
-                                                                                      L.t, L.u, L.v, L.occ, L.err);
-        else
-            k_trace_walk_ww<W, ANY, STACK, false><<<(unsigned)blocks, threads, 0, s>>>(tr, rays, n, nullptr, L.prim,
-                                                                                       L.t, L.u, L.v, L.occ, L.err);
-        return cudaGetLastError();
-    }
-    if (L.tuning.schedule == kSchedulePersistent && !L.n_dev && !STATS) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        int64_t blocks = (int64_t)(sms < 1 ? 1 : sms) * 9;  // 9 resident blocks of 128 per SM
-        const int64_t needed = (n + threads - 1) / threads;
-        if (blocks > needed) blocks = needed;
-        const int refill = L.tuning.refill_threshold < 1 ? 1 : (L.tuning.refill_threshold > 32 ? 32 : L.tuning.refill_threshold);
-        cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(unsigned long long), s);
-        if (e != cudaSuccess) return e;
-        k_trace_walk_persistent<W, ANY, STACK, false><<<(unsigned)blocks, threads, 0, s>>>(
-            tr, rays, n, L.counter, refill, nullptr, L.prim, L.t, L.u, L.v, L.occ, L.err);
-        return cudaGetLastError();
-    }
-    if (L.tuning.schedule == kSchedulePersistent && !L.n_dev) {
-        int dev = 0, sms = 0, blocks_per_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_trace_fp32_persistent<W, ANY, STACK, STATS>,
-                                                      threads, 0);
-        if (blocks_per_sm < 1) blocks_per_sm = 1;
-        if (sms < 1) sms = 1;
-        int64_t blocks = (int64_t)sms * blocks_per_sm;
-        const int64_t needed = (n + threads - 1) / threads;
-        if (blocks > needed) blocks = needed;
-        const int refill = L.tuning.refill_threshold < 1 ? 1 : (L.tuning.refill_threshold > 32 ? 32 : L.tuning.refill_threshold);
-        cudaError_t e = cudaMemsetAsync(L.counter, 0, sizeof(unsigned long long), s);
-        if (e != cudaSuccess) return e;
-        k_trace_fp32_persistent<W, ANY, STACK, STATS><<<(unsigned)blocks, threads, 0, s>>>(
-            tr, rays, n, L.counter, refill, L.prim, L.t, L.u, L.v, L.occ, L.err, L.stats);
-    } else if (STATS) {
-        const int64_t blocks = (n + threads - 1) / threads;
-        k_trace_fp32<W, ANY, STACK, STATS><<<(unsigned)blocks, threads, 0, s>>>(tr, rays, n, L.prim, L.t, L.u, L.v,
-                                                                                L.occ, L.err, L.stats, L.n_dev);
-    } else {
-        const int64_t blocks = (n + threads - 1) / threads;
-        k_trace_walk<W, ANY, STACK, false><<<(unsigned)blocks, threads, 0, s>>>(tr, rays, n, L.prim, L.t, L.u, L.v,
-                                                                               L.occ, L.err, L.n_dev, nullptr);
-    }
-    return cudaGetLastError();
+    return L.q8 ? launch_walk<W, ANY, STACK, true>(L, tr, rays, n, nullptr, L.counter, s)
+                : launch_walk<W, ANY, STACK, false>(L, tr, rays, n, nullptr, L.counter, s);
 }
 
 template <int W, bool ANY, bool STATS>

@@ -69,7 +69,7 @@ __device__ __forceinline__ float root_intersect(const RayState& r, const float* 
         if (r.d[a] < 0.00001f && r.d[a] > -0.00001f) {
             if (r.o[a] > hi[a] || r.o[a] < lo[a]) return -1.0f;
         } else {
-            const float ood = __frcp_rn(r.d[a]);
+            const float ood = r.rcp[a];  // 1/d: d is not clamped here (ray_setup)
             float t1 = __fmul_rn(__fsub_rn(hi[a], r.o[a]), ood);
             float t2 = __fmul_rn(__fsub_rn(lo[a], r.o[a]), ood);
             if (t1 > t2) {

@@ -9,16 +9,16 @@
 
 namespace sg {
 
-constexpr int kScheduleThreadPerRay = 0;  // one ray per thread for the whole launch
-constexpr int kSchedulePersistent = 1;    // persistent warps refilling idle lanes
-constexpr int kScheduleWhileWhile = 2;    // warp alternates interior and leaf phases
-constexpr int kScheduleSpeculative = 3;   // while-while, lanes keep descending past their first leaf
-constexpr int kScheduleSorted = 4;        // one ray per thread, rays taken in the order of a coherence key
-constexpr int kScheduleAuto = 5;          // sorted for large closest-hit batches, else thread per ray
+constexpr int kScheduleThreadPerRay = 0;  // rays taken in batch order
+constexpr int kSchedulePersistent = 1;    // the same, refilling at tuning.refill_threshold idle lanes
+constexpr int kScheduleWhileWhile = 2;    // as 0
+constexpr int kScheduleSpeculative = 3;   // as 0
+constexpr int kScheduleSorted = 4;        // rays taken in the order of a coherence key
+constexpr int kScheduleAuto = 5;          // sorted for large closest-hit batches, else batch order
 
 struct TraceTuning {
     int schedule = kScheduleAuto;
-    int refill_threshold = 8;  // idle lanes of a warp that trigger a refill (1..32)
+    int refill_threshold = 8;  // persistent schedule: idle lanes of a warp that trigger a refill (1..32)
 };
 
 struct TraceLaunch {
@@ -33,8 +33,9 @@ struct TraceLaunch {
     uint8_t* occ = nullptr;
     int* err = nullptr;
     unsigned long long* stats = nullptr;  // non-null: also accumulate SORT's traversal counters
-    unsigned long long* counter = nullptr;  // persistent schedule: ray counter, zeroed on the stream first
-    const int* n_dev = nullptr;  // if set, the batch is min(n, *n_dev) (one-ray-per-thread kernel)
+    unsigned* counter = nullptr;  // zero when the launch starts: warps take rays from it (null: the launch finds its own)
+    bool scratch = true;          // the launch may take stream-ordered scratch from the library's pool
+    const int* n_dev = nullptr;   // if set, the batch is min(n, *n_dev); large ones want a counter
     bool q8 = false;             // interior nodes in the 8-bit format
 };
 
