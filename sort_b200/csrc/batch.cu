@@ -5,20 +5,19 @@
 // The group's batches form one ray sequence (batch after batch, in table
 // order). A warp claims as many consecutive rays of it as it has idle lanes,
 // each lane finds its ray's batch by its position in that sequence, loads the
-// ray from the batch's planes and traverses its batch's tree with the same
-// per-ray traversal as the single-batch kernels (traversal.cuh), so every hit
-// is the one sg_trace_closest / sg_trace_any returns for that batch alone.
-// Like the persistent single-batch schedule, a warp refills once `refill`
-// lanes are idle (ray compaction between traversal steps).
+// ray from the batch's planes and traverses its batch's tree with the walk of
+// the single-batch kernels (warp_walk.cuh), so every hit is the one
+// sg_trace_closest / sg_trace_any returns for that batch alone. A warp refills
+// once `refill` lanes are idle.
 //
-// Each finished ray is counted against its batch (one atomic per batch per
-// warp step); the warp that finishes a batch's last ray stamps the batch's
-// completion time. A run may carry a time budget: once it has passed, warps
+// Finished rays are written and counted against their batch when their warp
+// refills (one atomic per batch and refill); the warp that counts a batch's
+// last ray stamps the batch's completion time. A run may carry a time budget: once it has passed, warps
 // stop claiming rays, finish the ones they hold and the run reports the cut.
 #include <cuda_runtime.h>
 
 #include "batch_kernels.h"
-#include "traversal.cuh"
+#include "warp_walk.cuh"
 
 namespace sg {
 
@@ -65,87 +64,89 @@ __device__ __forceinline__ void count_finished(bool fin, int b, const BatchArgs&
     }
 }
 
-// Held to 1,152 resident threads per SM (56 registers, nine blocks of 128):
-// with the traversal in RayWalk, batched_31m runs at 1,903 Mrays/s there
-// against 1,868 at 1,024 threads (64 registers) and 1,873 at 896 (72).
-template <int W, bool ANY, int STACK, int BLOCK, bool Q8>
-__global__ void __launch_bounds__(BLOCK, 1152 / BLOCK) k_trace_batches(BatchArgs a) {
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    const GroupDesc g = a.header->groups[a.group];
-    const int refill = a.header->refill;
-    const long long budget = a.header->budget_ns;
-    const BatchDesc* __restrict__ bt = a.batches + g.first;
-    RayWalk<W, ANY, STACK, Q8> tv;
-    uint2 stk[STACK];
-    DevTree tr;
-    tr.nodes = nullptr;
-    tr.tris = nullptr;
-    int b = 0;       // this lane's batch within the group
-    int64_t j = 0;   // its ray within that batch
-    bool alive = false;
-    bool drained = false;  // warp-uniform: nothing left to claim
-    if (g.count <= 0) return;
-    for (;;) {
-        const unsigned idle = __ballot_sync(0xffffffffu, !alive);
-        if (idle != 0 && !drained) {
-            unsigned long long base = 0;
-            if (lane == 0) {
-                if (budget > 0 && (long long)(global_ns() - a.state->start_ns) > budget) {
-                    atomicOr(&a.state->status, kBatchBudgetCut);
-                    base = (unsigned long long)g.total;
-                } else {
-                    base = atomicAdd(&a.state->counter[a.group], (unsigned long long)__popc(idle));
-                }
+// The walk's shared state with, per lane, its ray's batch and index there.
+struct BatchShared : WalkSharedMulti {
+    int64_t index[32];
+};
+
+template <bool ANY>
+struct BatchJob {
+    const BatchArgs& a;
+    const BatchDesc* __restrict__ bt;
+    int first, count;
+    int64_t total;
+    long long budget;
+    unsigned lanes;  // lanes that claim rays: a group of fewer rays than the grid has lanes is
+                     // claimed in equal shares, one per warp, so that it spreads over every SM
+    int b;           // this lane's batch within the group (its last one: the next search's hint)
+    bool drained;    // warp-uniform: nothing left to claim
+
+    __device__ __forceinline__ DevTree tree() const { return DevTree{}; }
+    __device__ __forceinline__ bool more() const { return !drained; }
+    __device__ __forceinline__ bool take(bool, unsigned mask, int lane, WalkSharedMulti* sh, RayState& r,
+                                         DevTree& tr) {
+        mask &= lanes;
+        unsigned long long base = 0;
+        if (lane == 0) {
+            if (budget > 0 && (long long)(global_ns() - a.state->start_ns) > budget) {
+                atomicOr(&a.state->status, kBatchBudgetCut);
+                base = (unsigned long long)total;
+            } else {
+                base = atomicAdd(&a.state->counter[a.group], (unsigned long long)__popc(mask));
             }
-            base = __shfl_sync(0xffffffffu, base, 0);
-            if ((int64_t)base >= g.total) drained = true;
-            bool fin = false;
-            if (!alive) {
-                const int64_t idx = (int64_t)base + __popc(idle & lt_mask);
-                if (idx < g.total) {
-                    b = find_batch(bt, g.count, idx, b);
-                    const float* p = bt[b].rays;
-                    const int64_t stride = __ldg(&bt[b].stride);
-                    j = idx - __ldg(&bt[b].start);
-                    p += j;
-                    tv.r.o[0] = __ldg(p);
-                    tv.r.o[1] = __ldg(p + stride);
-                    tv.r.o[2] = __ldg(p + 2 * stride);
-                    tv.r.d[0] = __ldg(p + 3 * stride);
-                    tv.r.d[1] = __ldg(p + 4 * stride);
-                    tv.r.d[2] = __ldg(p + 5 * stride);
-                    tv.r.tmin = __ldg(p + 6 * stride);
-                    tv.r.tmax = __ldg(p + 7 * stride);
-                    tr = a.trees[__ldg(&bt[b].tree)];
-                    alive = tv.begin(tr);
-                    if (!alive) {
-                        tv.finish(tr, j, bt[b].prim, bt[b].t, bt[b].u, bt[b].v, bt[b].occ);
-                        fin = true;
-                    }
-                }
-            }
-            count_finished(fin, b, a, g.first, lane);
         }
-        const unsigned busy0 = __ballot_sync(0xffffffffu, alive);
-        if (busy0 == 0) {
-            if (drained) break;
-            continue;
-        }
-        // Traverse until enough lanes are idle to be worth refilling.
-        for (;;) {
-            bool fin = false;
-            if (alive && tv.step(tr, stk, &a.state->status)) {
-                tv.finish(tr, j, bt[b].prim, bt[b].t, bt[b].u, bt[b].v, bt[b].occ);
-                alive = false;
-                fin = true;
-            }
-            count_finished(fin, b, a, g.first, lane);
-            const unsigned busy = __ballot_sync(0xffffffffu, alive);
-            if (busy == 0) break;
-            if (!drained && 32 - __popc(busy) >= refill) break;
-        }
+        base = __shfl_sync(kFullWarp, base, 0);
+        if ((int64_t)base >= total || lanes != kFullWarp) drained = true;
+        const int64_t idx = (int64_t)base + __popc(mask & ((1u << lane) - 1u));
+        if (!((mask >> lane) & 1u) || idx >= total) return false;
+        b = find_batch(bt, count, idx, b);
+        const BatchDesc& d = bt[b];
+        const int64_t stride = __ldg(&d.stride), j = idx - __ldg(&d.start);
+        const float* p = d.rays + j;
+        r.o[0] = __ldg(p);
+        r.o[1] = __ldg(p + stride);
+        r.o[2] = __ldg(p + 2 * stride);
+        r.d[0] = __ldg(p + 3 * stride);
+        r.d[1] = __ldg(p + 4 * stride);
+        r.d[2] = __ldg(p + 5 * stride);
+        r.tmin = __ldg(p + 6 * stride);
+        r.tmax = __ldg(p + 7 * stride);
+        tr = a.trees[__ldg(&d.tree)];
+        sh->ray[lane] = 0;
+        static_cast<BatchShared*>(sh)->index[lane] = j;
+        return true;
     }
+    __device__ __forceinline__ void put(bool fin, int lane, const WalkSharedMulti* sh) const {
+        if (fin) {
+            const BatchDesc& d = bt[b];
+            const int64_t j = static_cast<const BatchShared*>(sh)->index[lane];
+            const int32_t prim = sh->prim[lane];
+            if constexpr (ANY) {
+                d.occ[j] = prim >= 0 ? 1 : 0;
+            } else {
+                d.prim[j] = prim;
+                d.t[j] = sh->t[lane];
+                if (d.u) d.u[j] = prim >= 0 ? sh->u[lane] : 0.0f;
+                if (d.v) d.v[j] = prim >= 0 ? sh->v[lane] : 0.0f;
+            }
+        }
+        count_finished(fin, b, a, first, (unsigned)lane);
+    }
+};
+
+// Held to 896 resident threads per SM (72 registers), as k_trace_walk. 24 batches
+// of 4k .. 1M rays over five scenes (10k .. 2M triangles, width 8): 2.22 -> 1.01
+// ms against one ray per lane with every ray written and counted as it ended.
+template <int W, bool ANY, int STACK, int BLOCK, bool Q8>
+__global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace_batches(const __grid_constant__ BatchArgs a) {
+    __shared__ BatchShared shared[BLOCK / 32];
+    const GroupDesc g = a.header->groups[a.group];
+    if (g.count <= 0) return;
+    const int64_t warps = (int64_t)gridDim.x * (BLOCK / 32), share = (g.total + warps - 1) / warps;
+    const unsigned lanes = share < 32 ? (1u << share) - 1u : kFullWarp;
+    BatchJob<ANY> job{a, a.batches + g.first, g.first, g.count, g.total, a.header->budget_ns, lanes, 0, false};
+    walk_rays<W, ANY, STACK, Q8, true>(job, &shared[threadIdx.x >> 5], (int)(threadIdx.x & 31u), a.header->refill,
+                                       &a.state->status);
 }
 
 __global__ void k_batch_begin(const RunHeader* __restrict__ h, const BatchDesc* __restrict__ batches,

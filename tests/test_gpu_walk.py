@@ -97,3 +97,30 @@ def test_captured_and_concurrent_launches(port):
     torch.cuda.synchronize()
     for h in [captured] + results:
         assert np.array_equal(h.prim.cpu().numpy(), want[0]) and same_bits(h.t.cpu().numpy(), want[1])
+
+
+@pytest.mark.parametrize("sizes", [(1,), (33, 0, 5), (4_000, 7), (140_001, 1, 3)])
+def test_batch_groups_smaller_and_larger_than_the_grid(sizes):
+    """A group of fewer rays than the grid has lanes is claimed in equal shares,
+    a larger one from its counter: each batch's answers are its own launch's."""
+    from sort_b200 import Batch, Batcher, scenes
+    accs = []
+    for width, seed in ((8, 47), (4, 48)):
+        accs.append(accel(width))
+        accs[-1].Build(scenes.sphere_field(16, 2, seed=seed))
+    pool = torch.from_numpy(scenes.random_rays(150_000, seed=49)).cuda()
+    batches = [Batch(a, pool[:, k:k + n], any=q) for a in accs for q in (False, True) for k, n in enumerate(sizes)]
+    batcher = Batcher(max_batches=32)
+    for _ in range(2):
+        batcher.run(batches)
+        done = batcher.wait()
+        assert (done[: len(batches)] >= 0).all()
+        for b in batches:
+            if b.rays.shape[1] == 0:
+                continue
+            if b.any:
+                assert torch.equal(b.occluded, b.accel.GetAttenuation(b.rays))
+            else:
+                h = b.accel.GetIntersect(b.rays)
+                assert torch.equal(b.hits.prim, h.prim) and torch.equal(b.hits.t.view(torch.int32), h.t.view(torch.int32))
+    batcher.Release()
