@@ -31,7 +31,7 @@
 
 #include "pt_common.cuh"
 #include "serve_kernels.h"
-#include "traversal.cuh"
+#include "warp_walk.cuh"
 
 namespace sg {
 namespace {
@@ -120,38 +120,83 @@ __global__ void k_srv_regen(SrvBuffers b, float* __restrict__ qray, int* __restr
 }
 
 __global__ void k_srv_settle(SrvBuffers b) {
-    if (threadIdx.x == 0 && blockIdx.x == 0 && b.counters->head > b.counters->tail)
-        b.counters->head = b.counters->tail;
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    if (b.counters->head > b.counters->tail) b.counters->head = b.counters->tail;
+    b.counters->taken[0] = b.counters->taken[1] = 0;
 }
 
-// One ray per thread over a queue of rays from many scenes. Held to 9 blocks
-// of 128 per SM (56 registers; 12 bytes spilled for width-8 FP32 trees):
-// serve_27m's closed loop runs 3.6% faster than at the compiler's 60-80
-// registers.
-// Rays begin (null: 0) .. count - 1 of the queue.
-template <int W, bool ANY, int STACK, bool Q8>
-__global__ void __launch_bounds__(128, 9) k_srv_trace(const SrvScene* __restrict__ scenes, const float* __restrict__ ray,
-                                                   const int* __restrict__ scene_of, int cap,
-                                                   const int* __restrict__ begin, const int* __restrict__ count,
-                                                   int32_t* __restrict__ prim, float* __restrict__ t,
-                                                   uint8_t* __restrict__ occ, int* __restrict__ err) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *count || (begin && i < *begin)) return;
-    const DevTree tr = scenes[scene_of[i]].tree;
-    const DevRays rays{ray, ray + cap, ray + 2 * cap, ray + 3 * cap, ray + 4 * cap, ray + 5 * cap, ray + 6 * cap,
-                       ray + 7 * cap};
-    RayWalk<W, ANY, STACK, Q8> tv;
-    uint2 stk[STACK];
-    if (tv.start(tr, rays, i))
-        while (!tv.step(tr, stk, err)) {
+// Rays begin (null: 0) .. count - 1 of a queue of rays from many scenes, with
+// the walk of the single-batch kernels (warp_walk.cuh). taken (zero at launch)
+// counts the rays the warps have taken; a queue shorter than the grid's lanes
+// is shared out evenly.
+struct SrvJob {
+    const SrvScene* __restrict__ scenes;
+    const float* __restrict__ ray;
+    const int* __restrict__ scene_of;
+    int cap, begin, n;
+    int32_t* __restrict__ prim;
+    float* __restrict__ t;
+    uint8_t* __restrict__ occ;
+    unsigned* taken;
+    unsigned lanes;  // lanes that take rays
+    bool drained;    // warp-uniform
+
+    __device__ __forceinline__ DevTree tree() const { return DevTree{}; }
+    __device__ __forceinline__ bool more() const { return !drained; }
+    __device__ __forceinline__ bool take(bool, unsigned mask, int lane, WalkSharedMulti* sh, RayState& r, DevTree& tr) {
+        mask &= lanes;
+        unsigned base = 0;
+        if (lane == 0) base = atomicAdd(taken, (unsigned)__popc(mask));
+        base = __shfl_sync(kFullWarp, base, 0);
+        if (base >= (unsigned)n || lanes != kFullWarp) drained = true;
+        const unsigned k = base + (unsigned)__popc(mask & ((1u << lane) - 1u));
+        if (!((mask >> lane) & 1u) || k >= (unsigned)n) return false;
+        const int i = begin + (int)k;
+        tr = scenes[scene_of[i]].tree;
+        sh->ray[lane] = (uint32_t)i;
+        r.o[0] = ray[i];
+        r.o[1] = ray[cap + i];
+        r.o[2] = ray[2 * cap + i];
+        r.d[0] = ray[3 * cap + i];
+        r.d[1] = ray[4 * cap + i];
+        r.d[2] = ray[5 * cap + i];
+        r.tmin = ray[6 * cap + i];
+        r.tmax = ray[7 * cap + i];
+        return true;
+    }
+    __device__ __forceinline__ void put(bool fin, int lane, const WalkSharedMulti* sh) const {
+        if (!fin) return;
+        const uint32_t i = sh->ray[lane] & kWalkRayMask;
+        if (occ) {
+            occ[i] = sh->prim[lane] >= 0 ? 1 : 0;
+        } else {
+            prim[i] = sh->prim[lane];
+            t[i] = sh->t[lane];
         }
-    tv.finish(tr, i, prim, t, nullptr, nullptr, occ);
+    }
+};
+
+// 7 blocks of 128 per SM (72 registers), as k_trace_walk.
+constexpr int kSrvTraceBlocks = 7;
+template <int W, bool ANY, int STACK, bool Q8>
+__global__ void __launch_bounds__(kWalkThreads, kSrvTraceBlocks)
+    k_srv_trace(const SrvScene* __restrict__ scenes, const float* __restrict__ ray, const int* __restrict__ scene_of,
+                int cap, const int* __restrict__ begin, const int* __restrict__ count, int32_t* __restrict__ prim,
+                float* __restrict__ t, uint8_t* __restrict__ occ, unsigned* taken, int* __restrict__ err) {
+    __shared__ WalkSharedMulti shared[kWalkWarps];
+    const int first = begin ? *begin : 0, n = *count - first;
+    if (n <= 0) return;
+    const int warps = (int)gridDim.x * kWalkWarps, share = (n + warps - 1) / warps;
+    SrvJob job{scenes, ray,   scene_of, cap, first, n, prim, t, ANY ? occ : nullptr, taken,
+               share < 32 ? (1u << share) - 1u : kFullWarp, false};
+    walk_rays<W, ANY, STACK, Q8, true>(job, &shared[threadIdx.x >> 5], (int)(threadIdx.x & 31u), 10, err);
 }
 
 __global__ void k_srv_shade(SrvBuffers b, const float* __restrict__ qray, const int* __restrict__ qslot,
                             const int* __restrict__ qscene, float* __restrict__ nray, int* __restrict__ nslot,
                             int* __restrict__ nscene) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q == 0) b.counters->taken[2] = 0;  // the side stream's last traversal is done, its next one follows
     if (q >= b.counters->queue[0]) return;
     const int C = (int)b.slots, SC = 2 * C;
     const int s = qslot[q];
@@ -283,9 +328,11 @@ cudaError_t enqueue_stack(const SrvBuffers& b, int iterations, const SrvStreams&
     const cudaStream_t s = st.main;
     const int C = (int)b.slots;
     const int pool_blocks = (C + kThreads - 1) / kThreads;
-    const int trace_blocks = (C + 127) / 128;
-    const int shadow_blocks = (2 * C + 127) / 128;
-    cudaError_t e = cudaSuccess;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    const int trace_blocks = (sms < 1 ? 1 : sms) * kSrvTraceBlocks;  // warps take rays until the queue is empty
     for (int it = 0; it < iterations; ++it) {
         const bool a_cur = (it % 2) == 0;  // even steps read queue A and write queue B
         float* cray = a_cur ? b.qa_ray : b.qb_ray;
@@ -302,9 +349,9 @@ cudaError_t enqueue_stack(const SrvBuffers& b, int iterations, const SrvStreams&
         }
         k_srv_regen<<<pool_blocks, kThreads, 0, s>>>(b, cray, cslot, cscene);
         k_srv_settle<<<1, 32, 0, s>>>(b);
-        k_srv_trace<W, false, STACK, Q8><<<trace_blocks, 128, 0, s>>>(
+        k_srv_trace<W, false, STACK, Q8><<<trace_blocks, kWalkThreads, 0, s>>>(
             b.scenes, cray, cscene, C, traced ? &b.counters->queue[3] : nullptr, &b.counters->queue[0], b.hit_prim,
-            b.hit_t, nullptr, b.err);
+            b.hit_t, nullptr, &b.counters->taken[0], b.err);
         if (traced && (e = cudaStreamWaitEvent(s, st.joined, 0)) != cudaSuccess) return e;
         k_srv_shade<<<pool_blocks, kThreads, 0, s>>>(b, cray, cslot, cscene, nray, nslot, nscene);
         if (st.side && it + 1 < iterations) {
@@ -315,12 +362,14 @@ cudaError_t enqueue_stack(const SrvBuffers& b, int iterations, const SrvStreams&
                 (e = cudaEventRecord(st.forked, s)) != cudaSuccess ||
                 (e = cudaStreamWaitEvent(st.side, st.forked, 0)) != cudaSuccess)
                 return e;
-            k_srv_trace<W, false, STACK, Q8><<<trace_blocks, 128, 0, st.side>>>(
-                b.scenes, nray, nscene, C, nullptr, &b.counters->queue[3], b.hit_prim, b.hit_t, nullptr, b.err);
+            k_srv_trace<W, false, STACK, Q8><<<trace_blocks, kWalkThreads, 0, st.side>>>(
+                b.scenes, nray, nscene, C, nullptr, &b.counters->queue[3], b.hit_prim, b.hit_t, nullptr,
+                &b.counters->taken[2], b.err);
             if ((e = cudaEventRecord(st.joined, st.side)) != cudaSuccess) return e;
         }
-        k_srv_trace<W, true, STACK, Q8><<<shadow_blocks, 128, 0, s>>>(
-            b.scenes, b.sq_ray, b.sq_scene, 2 * C, nullptr, &b.counters->queue[2], nullptr, nullptr, b.occ, b.err);
+        k_srv_trace<W, true, STACK, Q8><<<trace_blocks, kWalkThreads, 0, s>>>(
+            b.scenes, b.sq_ray, b.sq_scene, 2 * C, nullptr, &b.counters->queue[2], nullptr, nullptr, b.occ,
+            &b.counters->taken[1], b.err);
         k_srv_resolve<<<(2 * C + kThreads - 1) / kThreads, kThreads, 0, s>>>(b);
         k_srv_accumulate<<<pool_blocks, kThreads, 0, s>>>(b, cslot);
         k_srv_advance<<<1, 32, 0, s>>>(b);

@@ -60,6 +60,7 @@ struct SrvControl {
 struct SrvCounters {
     int queue[4];               // [0] current extension queue, [1] next, [2] shadow queue,
                                 // [3] continuation rays of the current queue already traced
+    unsigned taken[3];          // rays taken by the step's traversals: extension, shadow, continuations
     unsigned long long head;    // ring entries claimed
     unsigned long long tail;    // ring entries appended
     unsigned long long ext_rays, shadow_rays;
