@@ -526,8 +526,8 @@ def run_pathtrace(args):
                    "d2h_bytes_per_step": int(host_img.numel() * 4 / args.steps)},
            "clocks": clocks.summary(), "image_mean": [round(float(v), 5) for v in host_img.mean(dim=(0, 1))],
            **({"image_rmse": rmse_info} if rmse_info else {}),
-           # per sample: generate, flush + per bounce (extend, shade, shadow, resolve, accumulate, count)
-           "gpu_launches": args.steps * (2 + 6 * PT_DEPTH) + 2}
+           # per sample: generate, flush + per bounce (extend, shade, shadow, accumulate)
+           "gpu_launches": args.steps * (2 + 4 * PT_DEPTH) + 2}
     if rank == 0:
         print(json.dumps(out))
     pt.Release()
@@ -818,10 +818,12 @@ def run_serve(args):
         st1 = srv.stats()
         # the server's own kernels in the closed-loop run: per graph replay the admission pair, 8 per
         # bounce step and a continuation trace on the side stream for every step but the last; per
-        # solo wave a generate and a flush, 6 per bounce
+        # solo wave (of several samples where the frame is small) a generate and a flush, 4 per bounce
         spp_ = args.steps_per_poll
+        waves = sum(-(-spp // max(1, min(spp, min(args.path_slots, 1 << 20) // (w * h))))
+                    for _, w, h, spp, _ in reqs if spp >= 2) if st1["solo_waves"] > st0["solo_waves"] else 0
         launches0 = ((st1["graph_replays"] - st0["graph_replays"]) * (2 + 8 * spp_ + spp_ - 1)
-                     + (st1["solo_waves"] - st0["solo_waves"]) * (2 + 6 * PT_DEPTH))
+                     + waves * (2 + 4 * PT_DEPTH))
         fifo_rate = len(reqs) / fifo_span0
         rows = []
         for frac in args.loads:

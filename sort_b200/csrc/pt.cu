@@ -1,6 +1,6 @@
 // Wavefront path tracer with SORT's PathTracing estimator (integrator/pathtracing.cpp:44-258).
 //
-// One wave traces one sample for every pixel. Per bounce:
+// One wave traces one sample, of small frames several, for every pixel. Per bounce:
 //   extend   closest-hit traversal of the compacted ray queue (trace.cu);
 //   shade    for each hit: emission at the first vertex, next-event estimation
 //            with both of EvaluateDirect's samples (integratormethod.cpp:100-192:
@@ -10,9 +10,9 @@
 //            shadow rays and the next rays are appended to compacted queues with
 //            one atomic per warp;
 //   shadow   any-hit traversal of the shadow queue;
-//   resolve  unoccluded shadow contributions go to their path's two slots, and
-//            are added to the path's radiance in a fixed order; at the end of
-//            the wave each path's radiance is added to its pixel. Every sum has
+//   accumulate  each path's unoccluded shadow contributions are added to its
+//            radiance in a fixed order; at the end of the wave each path's
+//            radiance is added to its pixel, sample after sample. Every sum has
 //            one writer in a fixed order, so an image is bit-reproducible.
 // Shading follows SORT's ScatteringEvent frame (scatteringevent.cpp:42-59) and
 // BxDFs: Lambert (lambert.cpp:34-38), MicroFacetReflection with GGX and
@@ -39,37 +39,50 @@
 namespace sg {
 namespace {
 
-// Path p renders frame pixel p0 + p (a band of whole rows starts at p0).
-__global__ void k_generate(Cam cam, int width, int height, int p0, int n, uint2 key, uint32_t sample, Queue q,
-                           int cap, float* __restrict__ thr, int* __restrict__ count) {
+// A wave's paths: path p renders sample `sample` + p / n of frame pixel
+// p0 + p % n (a band of whole rows starts at p0).
+struct WavePixels {
+    int p0, n;
+    uint32_t sample;
+    __device__ __forceinline__ int pixel(int p, uint32_t& smp) const {
+        const int k = p < n ? 0 : p / n;
+        smp = sample + (uint32_t)k;
+        return p0 + (p - k * n);
+    }
+};
+
+__global__ void k_generate(Cam cam, int width, int height, WavePixels px, int paths, uint2 key, Queue q, int cap,
+                           float* __restrict__ thr, WaveCount* __restrict__ counts) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    put_ray(q.ray, cap, p, cam.eye, camera_dir(cam, width, height, p0 + p, key, sample), 0.0f, FLT_MAX);
+    if (p >= paths) return;
+    uint32_t sample;
+    const int pixel = px.pixel(p, sample);
+    put_ray(q.ray, cap, p, cam.eye, camera_dir(cam, width, height, pixel, key, sample), 0.0f, FLT_MAX);
     q.slot[p] = p;
     thr[p] = thr[cap + p] = thr[2 * cap + p] = 1.0f;          // throughput
     thr[3 * cap + p] = thr[4 * cap + p] = thr[5 * cap + p] = 0.0f;  // radiance of this sample
     if (p == 0) {
-        count[kCurrent] = n;
-        count[kExtendTaken] = 0;
+        counts[0] = WaveCount{paths, 0, 0, 0};
+        counts[1] = WaveCount{0, 0, 0, 0};
     }
 }
 
-__global__ void k_shade(PtDev sc, uint2 key, int p0, uint32_t sample, int bounce, int max_depth, Queue in, int cap,
-                        const int* __restrict__ in_count, const int32_t* __restrict__ hit_prim,
-                        const float* __restrict__ hit_t, Queue next, int* __restrict__ next_count, Queue shadow,
-                        int shadow_cap, int* __restrict__ shadow_count, float* __restrict__ thr,
-                        float* __restrict__ vis) {
+__global__ void k_shade(PtDev sc, uint2 key, WavePixels px, int bounce, int max_depth, Queue in, int cap,
+                        WaveCount* __restrict__ counts, const int32_t* __restrict__ hit_prim,
+                        const float* __restrict__ hit_t, Queue next, Queue shadow, int shadow_cap,
+                        float* __restrict__ thr, int* __restrict__ shadow_of) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= *in_count) return;
+    if (q == 0) counts[(bounce + 2) % kWaveCounts] = WaveCount{0, 0, 0, 0};
+    if (q >= counts[bounce % kWaveCounts].length) return;
     const int p = in.slot[q];
     const int prim = hit_prim[q];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) vis[k * cap + p] = 0.0f;  // this bounce's two shadow results
     Vertex v;
     if (prim >= 0) {
         const float3 o = f3(in.ray[q], in.ray[cap + q], in.ray[2 * cap + q]);
         const float3 d = f3(in.ray[3 * cap + q], in.ray[4 * cap + q], in.ray[5 * cap + q]);
-        v = shade_vertex(sc, key, (uint32_t)(p0 + p), sample, bounce, max_depth, o, d, prim, hit_t[q],
+        uint32_t sample;
+        const int pixel = px.pixel(p, sample);
+        v = shade_vertex(sc, key, (uint32_t)pixel, sample, bounce, max_depth, o, d, prim, hit_t[q],
                          f3(thr[p], thr[cap + p], thr[2 * cap + p]));
         if (v.emit) {
             thr[3 * cap + p] += v.Le.x;
@@ -85,59 +98,64 @@ __global__ void k_shade(PtDev sc, uint2 key, int p0, uint32_t sample, int bounce
     const bool s1 = v.s1, s2 = v.s2, cont = v.cont;
     const float3 X = v.X, wi1 = v.wi1, wi2 = v.wi2, c1 = v.c1, c2 = v.c2, wi_next = v.wi_next;
     const float len1 = v.len1, t2 = v.t2;
-    const int i1 = warp_append(shadow_count, s1);
+    int* shadow_count = &counts[bounce % kWaveCounts].shadow;
+    const int i1 = warp_append(shadow_count, s1);  // light-sample ray
+    shadow_of[p] = i1;
     if (i1 >= 0) {
         put_ray(shadow.ray, shadow_cap, i1, X, wi1, 0.01f, len1 - 0.01f);
-        shadow.slot[i1] = 2 * p;  // light-sample result
         shadow.contrib[i1] = c1.x;
         shadow.contrib[shadow_cap + i1] = c1.y;
         shadow.contrib[2 * shadow_cap + i1] = c1.z;
     }
-    const int i2 = warp_append(shadow_count, s2);
+    const int i2 = warp_append(shadow_count, s2);  // BSDF-sample ray
+    shadow_of[cap + p] = i2;
     if (i2 >= 0) {
         put_ray(shadow.ray, shadow_cap, i2, X, wi2, 0.001f, t2 - 0.001f);
-        shadow.slot[i2] = 2 * p + 1;  // BSDF-sample result
         shadow.contrib[i2] = c2.x;
         shadow.contrib[shadow_cap + i2] = c2.y;
         shadow.contrib[2 * shadow_cap + i2] = c2.z;
     }
-    const int in_next = warp_append(next_count, cont);
+    const int in_next = warp_append(&counts[(bounce + 1) % kWaveCounts].length, cont);
     if (in_next >= 0) {
         put_ray(next.ray, cap, in_next, X, wi_next, 0.0001f, FLT_MAX);
         next.slot[in_next] = p;
     }
 }
 
-// Unoccluded shadow rays leave their contribution in their path's slot (one
-// writer per slot, so the sums below do not depend on scheduling).
-__global__ void k_resolve(Queue shadow, int shadow_cap, const int* __restrict__ count, const uint8_t* __restrict__ occ,
-                          float* __restrict__ vis, int cap) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= *count || occ[i]) return;
-    const int code = shadow.slot[i];
-    const int p = code >> 1, which = code & 1;
-    vis[(3 * which + 0) * cap + p] = shadow.contrib[i];
-    vis[(3 * which + 1) * cap + p] = shadow.contrib[shadow_cap + i];
-    vis[(3 * which + 2) * cap + p] = shadow.contrib[2 * shadow_cap + i];
-}
-
-// EvaluateDirect's two terms are added to the path's radiance in SORT's order
-// (light sample, then BSDF sample), for every path shaded this bounce.
-__global__ void k_accumulate(Queue in, const int* __restrict__ in_count, const float* __restrict__ vis,
-                             float* __restrict__ thr, int cap) {
+// EvaluateDirect's two terms (light sample, then BSDF sample; an occluded or
+// absent ray's is zero) are added to the path's radiance in SORT's order, for
+// every path shaded this bounce. Adding two zeros would change nothing, so such
+// paths are passed over. Also counts the bounce's rays.
+__global__ void k_accumulate(Queue in, const WaveCount* __restrict__ count, const int* __restrict__ shadow_of,
+                             const uint8_t* __restrict__ occ, const float* __restrict__ contrib, int shadow_cap,
+                             float* __restrict__ thr, int cap, unsigned long long* __restrict__ totals) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= *in_count) return;
+    if (q == 0) {  // waves of two samples may count at once
+        atomicAdd(&totals[0], (unsigned long long)count->length);
+        atomicAdd(&totals[1], (unsigned long long)count->shadow);
+    }
+    if (q >= count->length) return;
     const int p = in.slot[q];
+    const int i1 = shadow_of[p], i2 = shadow_of[cap + p];
+    const bool lit1 = i1 >= 0 && !occ[i1], lit2 = i2 >= 0 && !occ[i2];
+    if (!lit1 && !lit2) return;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) thr[(3 + c) * cap + p] += vis[c * cap + p] + vis[(3 + c) * cap + p];
+    for (int c = 0; c < 3; ++c)
+        thr[(3 + c) * cap + p] +=
+            (lit1 ? contrib[c * shadow_cap + i1] : 0.0f) + (lit2 ? contrib[c * shadow_cap + i2] : 0.0f);
 }
 
-// End of a wave: each pixel's sample radiance goes into the image (one writer).
-__global__ void k_flush(const float* __restrict__ thr, int cap, int n, float* __restrict__ image) {
+// End of a wave: each pixel's sample radiances go into the image, sample after
+// sample (one writer).
+__global__ void k_flush(const float* __restrict__ thr, int cap, int n, int samples, float* __restrict__ image) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) image[3 * p + c] += thr[(3 + c) * cap + p];
+    for (int c = 0; c < 3; ++c) {
+        float sum = image[3 * p + c];
+        for (int k = 0; k < samples; ++k) sum += thr[(3 + c) * cap + k * n + p];
+        image[3 * p + c] = sum;
+    }
 }
 
 __global__ void k_scale(float* __restrict__ image, int n, float s) {
@@ -148,15 +166,6 @@ __global__ void k_scale(float* __restrict__ image, int n, float s) {
 __global__ void k_zero(float* __restrict__ image, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) image[i] = 0.0f;
-}
-
-// Adds this bounce's queue lengths (extension rays, shadow rays) to the totals.
-__global__ void k_count_rays(const int* __restrict__ extension, const int* __restrict__ shadow,
-                             unsigned long long* __restrict__ totals) {
-    if (threadIdx.x == 0) {  // waves of two samples may count at once
-        atomicAdd(&totals[0], (unsigned long long)*extension);
-        atomicAdd(&totals[1], (unsigned long long)*shadow);
-    }
 }
 
 }  // namespace
@@ -173,8 +182,8 @@ struct sg_pt_scene {
     void* d_buf = nullptr;
     size_t buf_bytes = 0;
     unsigned long long* d_totals = nullptr;  // rays traced by the last render: extension, shadow
-    // kInFlight samples are in flight at once, each with its own buffers:
-    // sample k runs on the caller's stream (k % kInFlight == 0) or on
+    // kInFlight waves are in flight at once, each with its own buffers:
+    // wave k runs on the caller's stream (k % kInFlight == 0) or on
     // extra[k % kInFlight], its shadow rays on side[k % kInFlight]
     // (pt_wave.h); the events order the hand-offs and the image additions.
     // Made by the first render.
@@ -342,84 +351,71 @@ cudaError_t pt_scale(float* image, int64_t n, float s, cudaStream_t st) {
 }
 
 cudaError_t pt_wave(const PtDev& dev, const TraceLaunch& base_in, const DevTree& tree, const Cam& cam, int width,
-                    int height, int p0, int n, uint2 key, int sample, int max_depth, const PtWave& w, float* image,
-                    cudaStream_t s) {
+                    int height, int p0, int n, uint2 key, int sample, int samples, int max_depth, const PtWave& w,
+                    float* image, cudaStream_t s) {
     const int cap = w.cap, scap = 2 * w.cap;
-    if (n <= 0 || n > cap) return cudaErrorInvalidValue;
+    if (n <= 0 || samples <= 0 || (int64_t)n * samples > cap) return cudaErrorInvalidValue;
+    const int paths = n * samples;
     TraceLaunch base = base_in;
     base.tuning.schedule = kScheduleThreadPerRay;  // queue lengths live on the device
     Queue qa{w.qa_ray, w.qa_slot, nullptr}, qb{w.qb_ray, w.qb_slot, nullptr};
-    const Queue sq{w.sq_ray, w.sq_slot, w.sq_contrib};
-    int* counters = w.counters;
+    const Queue sq{w.sq_ray, nullptr, w.sq_contrib};
+    const WavePixels px{p0, n, (uint32_t)sample};
     const int threads = 256;
-    const int blocks = (n + threads - 1) / threads;
+    const int blocks = (paths + threads - 1) / threads;
     cudaError_t e = cudaSuccess;
     Queue* cur = &qa;
     Queue* nxt = &qb;
-    auto closest = [&](const Queue* q) {
+    auto closest = [&](const Queue* q, WaveCount* count) {
         DevRays r{q->ray,           q->ray + cap,     q->ray + 2 * cap, q->ray + 3 * cap,
                   q->ray + 4 * cap, q->ray + 5 * cap, q->ray + 6 * cap, q->ray + 7 * cap};
         TraceLaunch Lc = base;
         Lc.any = false;
         Lc.prim = w.hit_prim;
         Lc.t = w.hit_t;
-        Lc.n_dev = &counters[kCurrent];
-        Lc.counter = reinterpret_cast<unsigned*>(&counters[kExtendTaken]);
-        return launch_trace_fp32(Lc, tree, r, (int64_t)cap, s);
+        Lc.n_dev = &count->length;
+        Lc.counter = &count->taken;
+        return launch_trace_fp32(Lc, tree, r, (int64_t)paths, s);
     };
-    // Shadow rays, their results and the path radiance of bounce `cur` on
-    // stream t; `shaded` is the length of the bounce's extension queue.
-    auto shadows = [&](const Queue* q, const int* shaded, cudaStream_t t) {
+    // Shadow rays of bounce `cur` and its paths' radiance on stream t.
+    auto shadows = [&](const Queue* q, WaveCount* count, cudaStream_t t) {
         DevRays sr{sq.ray,            sq.ray + scap,     sq.ray + 2 * scap, sq.ray + 3 * scap,
                    sq.ray + 4 * scap, sq.ray + 5 * scap, sq.ray + 6 * scap, sq.ray + 7 * scap};
         TraceLaunch La = base;
         La.any = true;
         La.occ = w.occ;
-        La.n_dev = &counters[kShadow];
-        La.counter = reinterpret_cast<unsigned*>(&counters[kShadowTaken]);
-        cudaError_t r = launch_trace_fp32(La, tree, sr, (int64_t)scap, t);
+        La.n_dev = &count->shadow;
+        La.counter = &count->shadow_taken;
+        cudaError_t r = launch_trace_fp32(La, tree, sr, 2 * (int64_t)paths, t);
         if (r != cudaSuccess) return r;
-        k_resolve<<<(scap + threads - 1) / threads, threads, 0, t>>>(sq, scap, &counters[kShadow], w.occ, w.vis, cap);
-        k_accumulate<<<blocks, threads, 0, t>>>(*q, shaded, w.vis, w.thr, cap);
-        k_count_rays<<<1, 32, 0, t>>>(shaded, &counters[kShadow], w.totals);
+        k_accumulate<<<blocks, threads, 0, t>>>(*q, count, w.shadow_of, w.occ, sq.contrib, scap, w.thr, cap, w.totals);
         return cudaGetLastError();
     };
-    k_generate<<<blocks, threads, 0, s>>>(cam, width, height, p0, n, key, (uint32_t)sample, *cur, cap, w.thr,
-                                          counters);
-    if ((e = closest(cur)) != cudaSuccess) return e;
+    k_generate<<<blocks, threads, 0, s>>>(cam, width, height, px, paths, key, *cur, cap, w.thr, w.counts);
+    if ((e = closest(cur, &w.counts[0])) != cudaSuccess) return e;
     for (int bounce = 0; bounce < max_depth; ++bounce) {
-        if ((e = cudaMemsetAsync(&counters[kNext], 0, (kShadowTaken - kNext + 1) * sizeof(int), s)) != cudaSuccess) return e;
-        k_shade<<<blocks, threads, 0, s>>>(dev, key, p0, (uint32_t)sample, bounce, max_depth, *cur, cap,
-                                           &counters[kCurrent], w.hit_prim, w.hit_t, *nxt, &counters[kNext], sq, scap,
-                                           &counters[kShadow], w.thr, w.vis);
-        const bool more = bounce + 1 < max_depth;
+        WaveCount* count = &w.counts[bounce % kWaveCounts];
+        k_shade<<<blocks, threads, 0, s>>>(dev, key, px, bounce, max_depth, *cur, cap, w.counts, w.hit_prim, w.hit_t,
+                                           *nxt, sq, scap, w.thr, w.shadow_of);
         if (!w.side) {
-            if ((e = shadows(cur, &counters[kCurrent], s)) != cudaSuccess) return e;
+            if ((e = shadows(cur, count, s)) != cudaSuccess) return e;
         } else {
             // The shadow rays of this bounce go to the side stream and run
             // beside the next bounce's extension rays; the next shading (which
-            // reuses the shadow queue, the path state and the counters) waits
-            // for them.
-            if ((e = cudaMemcpyAsync(&counters[kShaded], &counters[kCurrent], sizeof(int), cudaMemcpyDeviceToDevice, s)) !=
-                    cudaSuccess ||
-                (e = cudaEventRecord(w.shaded, s)) != cudaSuccess ||
+            // reuses the shadow queue and the path state) waits for them.
+            if ((e = cudaEventRecord(w.shaded, s)) != cudaSuccess ||
                 (e = cudaStreamWaitEvent(w.side, w.shaded, 0)) != cudaSuccess ||
-                (e = shadows(cur, &counters[kShaded], w.side)) != cudaSuccess ||
+                (e = shadows(cur, count, w.side)) != cudaSuccess ||
                 (e = cudaEventRecord(w.shadowed, w.side)) != cudaSuccess)
                 return e;
         }
-        // the next queue becomes the current one
-        if ((e = cudaMemcpyAsync(&counters[kCurrent], &counters[kNext], sizeof(int), cudaMemcpyDeviceToDevice, s)) !=
-            cudaSuccess)
+        std::swap(cur, nxt);  // the next queue becomes the current one
+        if (bounce + 1 < max_depth && (e = closest(cur, &w.counts[(bounce + 1) % kWaveCounts])) != cudaSuccess)
             return e;
-        Queue* t = cur;
-        cur = nxt;
-        nxt = t;
-        if (more && (e = closest(cur)) != cudaSuccess) return e;
         if (w.side && (e = cudaStreamWaitEvent(s, w.shadowed, 0)) != cudaSuccess) return e;
     }
     if (w.flush_after && (e = cudaStreamWaitEvent(s, w.flush_after, 0)) != cudaSuccess) return e;
-    k_flush<<<blocks, threads, 0, s>>>(w.thr, cap, n, image);
+    k_flush<<<(n + threads - 1) / threads, threads, 0, s>>>(w.thr, cap, n, samples, image);
     if (w.flush_done && (e = cudaEventRecord(w.flush_done, s)) != cudaSuccess) return e;
     return cudaGetLastError();
 }
@@ -459,16 +455,18 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
     } restore{prev};
     cudaStream_t s = (cudaStream_t)stream;
 
-    // Buffers, kInFlight times (samples in flight): two extension queues (rays +
-    // slots), hits, one shadow queue of 2 entries per path (rays + slots +
-    // contributions), occlusion flags, throughput, shadow results, the queue
-    // counters; then the shared ray totals.
-    const size_t cap = (size_t)P, scap = 2 * (size_t)P;
+    // Buffers of each wave in flight: two extension queues (rays + slots), hits,
+    // one shadow queue of 2 entries per path (rays + contributions), occlusion
+    // flags, throughput and radiance, shadow entries, counts; then the shared ray
+    // totals.
+    const int per_wave = sg::wave_samples(P, sg::kWavePaths, spp), waves = (spp + per_wave - 1) / per_wave;
+    const int in_flight = waves < sg::kInFlight ? waves : sg::kInFlight;
+    const size_t cap = (size_t)P * per_wave, scap = 2 * cap;
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
     const size_t qbytes = align(cap * 8 * 4) + align(cap * 4);
-    const size_t set = 2 * qbytes + align(cap * 4) * 2 + align(scap * 8 * 4) + align(scap * 4) +
-                       align(scap * 3 * 4) + align(scap) + align(cap * 6 * 4) + align(cap * 6 * 4) + align(sg::kWaveCounters * 4);
-    const size_t need = sg::kInFlight * set + align(16);
+    const size_t set = 2 * qbytes + align(cap * 4) * 2 + align(scap * 8 * 4) + align(scap * 3 * 4) + align(scap) +
+                       align(cap * 6 * 4) + align(cap * 2 * 4) + align(sg::kWaveCounts * sizeof(sg::WaveCount));
+    const size_t need = in_flight * set + align(16);
     if (ps->buf_bytes < need) {
         if (ps->d_buf) cudaFree(ps->d_buf);
         ps->d_buf = nullptr;
@@ -493,7 +491,7 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
     made = made && (ps->begun || cudaEventCreateWithFlags(&ps->begun, cudaEventDisableTiming) == cudaSuccess);
     if (!made) return sg::set_error(SG_ERR_CUDA, "render streams and events");
     sg::PtWave w[sg::kInFlight] = {};
-    for (int k = 0; k < sg::kInFlight; ++k) {
+    for (int k = 0; k < in_flight; ++k) {
         w[k].qa_ray = (float*)take(cap * 32);
         w[k].qa_slot = (int*)take(cap * 4);
         w[k].qb_ray = (float*)take(cap * 32);
@@ -501,12 +499,11 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
         w[k].hit_prim = (int32_t*)take(cap * 4);
         w[k].hit_t = (float*)take(cap * 4);
         w[k].sq_ray = (float*)take(scap * 32);
-        w[k].sq_slot = (int*)take(scap * 4);
         w[k].sq_contrib = (float*)take(scap * 12);
         w[k].occ = (uint8_t*)take(scap);
-        w[k].thr = (float*)take(cap * 24);  // throughput and radiance per path
-        w[k].vis = (float*)take(cap * 24);  // two shadow results per path
-        w[k].counters = (int*)take(sg::kWaveCounters * 4);
+        w[k].thr = (float*)take(cap * 24);    // throughput and radiance per path
+        w[k].shadow_of = (int*)take(cap * 8);  // two shadow queue entries per path
+        w[k].counts = (sg::WaveCount*)take(sg::kWaveCounts * sizeof(sg::WaveCount));
         w[k].cap = (int)cap;
         w[k].side = ps->side[k];
         w[k].shaded = ps->shaded[k];
@@ -529,18 +526,18 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
     if ((e = cudaEventRecord(ps->begun, s)) != cudaSuccess) return pt_fail(e);
     for (int k = 1; k < sg::kInFlight; ++k)
         if ((e = cudaStreamWaitEvent(ps->extra[k], ps->begun, 0)) != cudaSuccess) return pt_fail(e);
-    for (int sample = 0; sample < spp; ++sample) {
-        const int set = sample % sg::kInFlight;
+    for (int k = 0; k < waves; ++k) {
+        const int set = k % sg::kInFlight, first = k * per_wave;
         sg::PtWave& ws = w[set];
-        ws.flush_after = sample > 0 ? ps->flushed[(sample - 1) % sg::kInFlight] : nullptr;  // image sums in order
+        ws.flush_after = k > 0 ? ps->flushed[(k - 1) % sg::kInFlight] : nullptr;  // image sums in order
         const cudaStream_t on = set ? ps->extra[set] : s;
-        if ((e = sg::pt_wave(dev, base, tree, cam, width, height, p0, P, key, sample, max_depth, ws, image, on)) !=
-            cudaSuccess)
+        if ((e = sg::pt_wave(dev, base, tree, cam, width, height, p0, P, key, first, std::min(per_wave, spp - first),
+                             max_depth, ws, image, on)) != cudaSuccess)
             return pt_fail(e);
     }
     // Every stream's work is done before the scale: the last addition closes
-    // the chain, and every other stream's last sample precedes it.
-    if ((e = cudaStreamWaitEvent(s, ps->flushed[(spp - 1) % sg::kInFlight], 0)) != cudaSuccess) return pt_fail(e);
+    // the chain, and every other stream's last wave precedes it.
+    if ((e = cudaStreamWaitEvent(s, ps->flushed[(waves - 1) % sg::kInFlight], 0)) != cudaSuccess) return pt_fail(e);
     sg::k_scale<<<(img_n + threads - 1) / threads, threads, 0, s>>>(image, img_n, 1.0f / (float)spp);
     if ((e = cudaGetLastError()) != cudaSuccess) return pt_fail(e);
     return SG_OK;

@@ -1,7 +1,6 @@
-// One wave of the wavefront path tracer (pt.cu): one sample for every pixel
-// of a band, on caller-provided buffers. sg_pt_render_rows runs one wave per
-// sample on the render's own buffers; the render server (server.cpp) runs
-// waves on its idle path pool for a request that has the GPU to itself.
+// One wave of the wavefront path tracer (pt.cu): one or more samples for every
+// pixel of a band, on caller-provided buffers. sg_pt_render_rows runs its waves
+// on the render's own buffers; the render server (server.cpp) on its lanes'.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -13,34 +12,52 @@
 
 namespace sg {
 
-// Samples sg_pt_render keeps in flight, each on its own buffers and streams.
+// Waves sg_pt_render keeps in flight, each on its own buffers and streams.
 constexpr int kInFlight = 2;
 
-// Device buffers of a wave, with the layouts the server's pool uses: two
-// extension queues (8 floats per ray with stride cap, a path index per
-// entry), the hits (cap each), the shadow queue (stride 2 * cap, three
-// contribution planes) and its occlusion flags, per-path throughput and
-// radiance (6 * cap floats) and shadow results (6 * cap), the queue
-// counters (kWaveCounters) and two ray totals (extension, shadow).
-// Indices into PtWave::counters: queue lengths (the shaded queue's copy is for
-// the side stream) and the ray counters of the two traversals. kNext up to
-// kShadowTaken are zeroed together before each shading.
-enum { kCurrent = 0, kNext = 1, kShadow = 2, kExtendTaken = 3, kShadowTaken = 4, kShaded = 5, kWaveCounters = 6 };
+// Paths a wave of several samples holds at most: a small frame's samples share
+// waves, because a wave of few paths is bound by its chain of dependent launches
+// and by the latency of single rays, not by the work. A 161x91 frame of 4 spp
+// (four waves of 14,651 paths, then one of 58,604) went from 0.67 to
+// 0.285 ms, 480x270 at 16 spp from 6.03 to 2.16, a mix of 24 served renders
+// (64x36 to 960x540, 1 to 16 spp) from 28.7 to 12.9.
+constexpr int64_t kWavePaths = int64_t(1) << 20;
 
+// Samples per wave of a band of n pixels whose buffers hold cap paths.
+inline int wave_samples(int64_t n, int64_t cap, int spp) {
+    const int64_t most = (cap < kWavePaths ? cap : kWavePaths) / n;
+    return most < 1 ? 1 : (most > spp ? spp : (int)most);
+}
+
+// Queue lengths and ray counters of one bounce; bounce b uses entry b % 4 of the
+// wave's kWaveCounts entries. Shading bounce b appends to entry b + 1 and clears
+// entry b + 2, whose last users (bounce b - 2) are done, so that no memset or
+// copy stands between two kernels.
+struct WaveCount {
+    int length;                  // extension rays
+    int shadow;                  // shadow rays
+    unsigned taken, shadow_taken;  // rays taken by the two traversals
+};
+constexpr int kWaveCounts = 4;
+
+// Device buffers of a wave: two extension queues (8 floats per ray with stride
+// cap, a path index per entry), the hits (cap each), the shadow queue (stride
+// 2 * cap, three contribution planes) and its occlusion flags, per-path
+// throughput and radiance (6 * cap floats) and the path's two shadow queue
+// entries (2 * cap, -1: none), the counts and two ray totals (extension, shadow).
 struct PtWave {
     float* qa_ray;
     int* qa_slot;
     float* qb_ray;
     int* qb_slot;
     float* sq_ray;
-    int* sq_slot;
     float* sq_contrib;
     int32_t* hit_prim;
     float* hit_t;
     uint8_t* occ;
     float* thr;
-    float* vis;
-    int* counters;  // kWaveCounters, see the indices below
+    int* shadow_of;
+    WaveCount* counts;  // kWaveCounts
     unsigned long long* totals;
     int cap;
     // Optional: a second stream on which each bounce's shadow rays run beside
@@ -53,16 +70,17 @@ struct PtWave {
     cudaEvent_t flush_after, flush_done;
 };
 
-// Sample `sample` of pixels p0 .. p0 + n - 1 (n <= w.cap) of a width x height
-// frame: each pixel's radiance is added to image[3 * (p - p0) + c]; nothing is
-// zeroed or scaled. Every pixel draws the random numbers of its place in the
-// frame, so waves over bands and over whole frames give the same sums.
-// `base` is the scene's launch (scene_launch), `tree` its tree.
 // image[i] *= s for i < n (the 1/spp of a finished render), on stream st.
 cudaError_t pt_scale(float* image, int64_t n, float s, cudaStream_t st);
 
+// Samples sample .. sample + samples - 1 of pixels p0 .. p0 + n - 1 (n * samples
+// <= w.cap) of a width x height frame: each pixel's radiance is added to
+// image[3 * (p - p0) + c], sample after sample; nothing is zeroed or scaled.
+// Every pixel draws the random numbers of its place in the frame, so waves over
+// bands and over whole frames, of one sample or of several, give the same sums.
+// `base` is the scene's launch (scene_launch), `tree` its tree.
 cudaError_t pt_wave(const PtDev& dev, const TraceLaunch& base, const DevTree& tree, const Cam& cam, int width,
-                    int height, int p0, int n, uint2 key, int sample, int max_depth, const PtWave& w, float* image,
-                    cudaStream_t s);
+                    int height, int p0, int n, uint2 key, int sample, int samples, int max_depth, const PtWave& w,
+                    float* image, cudaStream_t s);
 
 }  // namespace sg

@@ -11,8 +11,8 @@
 //
 // Solo lanes: a multi-sample request of at least solo_pixels pixels waits for
 // one of the lanes (oldest first) and is rendered the way sg_pt_render
-// renders a frame, one wave per sample (pt_wave, on the lane's own buffers),
-// two samples in flight on the lane's streams, while the pool serves the
+// renders a frame, in waves of one or more samples (pt_wave, on the lane's own
+// buffers), two in flight on the lane's streams, while the pool serves the
 // other requests; the lane holding the oldest request uses the high-priority
 // streams. After its last wave the lane scales the image and the request
 // completes like a pool request. In the pool a pixel's samples run one after
@@ -131,12 +131,13 @@ struct sg_server {
     // pairs (sample k on [k % 2]), beside the pool's `stream`.
     struct Lane {
         int64_t id = -1;  // ticket in its solo phase
-        int next = 0;     // next sample to queue a wave for
+        int next = 0;     // next wave to queue
         int done = 0;     // waves finished
-        int last = 0;     // waves to run (spp)
+        int last = 0;     // waves to run
+        int samples = 1;  // samples per wave (wave_samples; 1 where a frame takes several bands)
         bool finishing = false;  // every wave queued (and the scale), or cancelled: waiting for `end`
         sg::PtWave w[2] = {};
-        // The waves and their shadow rays (pt_wave.h), [priority][sample % 2]:
+        // The waves and their shadow rays (pt_wave.h), [priority][wave % 2]:
         // the lane holding the oldest request queues its waves on the
         // high-priority streams, the others (and the pool) on normal ones.
         cudaStream_t stream[2][2] = {};
@@ -348,7 +349,8 @@ void start_solo(sg_server* S) {
             for (cudaStream_t t : pair) cudaStreamWaitEvent(t, L.ready, 0);
         L.id = id;
         L.next = L.done = 0;
-        L.last = t.req.spp;
+        L.samples = sg::wave_samples(int64_t(t.req.width) * t.req.height, L.w[0].cap, t.req.spp);
+        L.last = (t.req.spp + L.samples - 1) / L.samples;
         L.finishing = false;
     }
 }
@@ -431,6 +433,7 @@ sg_status pump_lane(sg_server* S, int l) {
     sg::SrvScene sc;
     sg::TraceLaunch base;
     bool end = false, oldest = true;
+    int spp = 1;
     {
         std::lock_guard<std::mutex> lk(S->mu);  // add_scene may grow the scene tables meanwhile
         const Ticket& t = S->tickets[L.id];
@@ -438,6 +441,7 @@ sg_status pump_lane(sg_server* S, int l) {
         sc = S->scenes[size_t(q.scene)];
         base = S->launches[size_t(q.scene)];
         end = S->stop || t.cancel;
+        spp = t.req.spp;
         for (const sg_server::Lane& o : S->lanes)  // an older request in another lane
             if (o.id >= 0 && o.id != L.id) {
                 const Ticket& u = S->tickets[o.id];
@@ -446,9 +450,9 @@ sg_status pump_lane(sg_server* S, int l) {
     }
     const int rows = std::max(1, L.w[0].cap / q.width);  // rows per band: a band fits the wave buffers
     while (!end && L.next < L.last && L.next - L.done < 2) {
-        // Sample k on buffer set and stream pair k % 2; its image additions
-        // wait for sample k - 1's.
-        const int k = L.next;
+        // Wave k on buffer set and stream pair k % 2; its image additions
+        // wait for wave k - 1's.
+        const int k = L.next, first = k * L.samples, samples = std::min(L.samples, spp - first);
         sg::PtWave w = L.w[k % 2];
         w.flush_after = k > 0 ? L.flushed[(k - 1) % 2] : nullptr;
         w.flush_done = L.flushed[k % 2];
@@ -458,15 +462,15 @@ sg_status pump_lane(sg_server* S, int l) {
         for (int y = 0; y < q.height && e == cudaSuccess; y += rows) {
             const int y1 = std::min(q.height, y + rows);
             const int p0 = y * q.width;
-            e = sg::pt_wave(sc.pt, base, sc.tree, q.cam, q.width, q.height, p0, (y1 - y) * q.width, q.key, k,
-                            q.max_depth, w, q.image + 3 * int64_t(p0), on);
+            e = sg::pt_wave(sc.pt, base, sc.tree, q.cam, q.width, q.height, p0, (y1 - y) * q.width, q.key,
+                            first, samples, q.max_depth, w, q.image + 3 * int64_t(p0), on);
         }
         if (e == cudaSuccess) e = cudaEventRecord(L.wave_done[k % 2], on);
         if (e != cudaSuccess) return fail(SG_ERR_CUDA, std::string("solo wave: ") + cudaGetErrorString(e));
         L.last_on = on;
         L.next++;
         std::lock_guard<std::mutex> lk(S->mu);
-        S->stats.solo_waves++;
+        S->stats.solo_waves += samples;
     }
     if (end || L.next == L.last) {
         // After the last wave, whose additions came after every earlier one's:
@@ -767,8 +771,8 @@ sg_status sg_server_create(const sg_server_opts* opts, sg_server** out) {
         // state, counters; then the ray totals every set adds to.
         S->lanes.resize(kSoloLanes);
         const size_t cap = C, scap = 2 * C;
-        const size_t parts[] = {cap * 32, cap * 4, cap * 32, cap * 4, cap * 4, cap * 4, scap * 32, scap * 4,
-                                scap * 12, scap, cap * 24, cap * 24, sg::kWaveCounters * 4};
+        const size_t parts[] = {cap * 32, cap * 4, cap * 32, cap * 4, cap * 4, cap * 4, scap * 32, scap * 12,
+                                scap, cap * 24, cap * 8, sg::kWaveCounts * sizeof(sg::WaveCount)};
         constexpr int kParts = int(sizeof(parts) / sizeof(parts[0]));
         size_t set = 0;
         for (size_t x : parts) set += align_up(x);
@@ -791,12 +795,11 @@ sg_status sg_server_create(const sg_server_opts* opts, sg_server** out) {
                 w.hit_prim = reinterpret_cast<int32_t*>(at[4]);
                 w.hit_t = reinterpret_cast<float*>(at[5]);
                 w.sq_ray = reinterpret_cast<float*>(at[6]);
-                w.sq_slot = reinterpret_cast<int*>(at[7]);
-                w.sq_contrib = reinterpret_cast<float*>(at[8]);
-                w.occ = reinterpret_cast<uint8_t*>(at[9]);
-                w.thr = reinterpret_cast<float*>(at[10]);
-                w.vis = reinterpret_cast<float*>(at[11]);
-                w.counters = reinterpret_cast<int*>(at[12]);
+                w.sq_contrib = reinterpret_cast<float*>(at[7]);
+                w.occ = reinterpret_cast<uint8_t*>(at[8]);
+                w.thr = reinterpret_cast<float*>(at[9]);
+                w.shadow_of = reinterpret_cast<int*>(at[10]);
+                w.counts = reinterpret_cast<sg::WaveCount*>(at[11]);
                 w.cap = int(cap);
                 for (int pr = 0; pr < 2 && e == cudaSuccess; ++pr) {
                     const int level = pr == 0 ? greatest : least;
