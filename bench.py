@@ -373,7 +373,6 @@ def run_ours(args):
                 traffic = tj.get("dram_bytes_per_launch")
 
     if rank == 0:
-        sorted_schedule = n >= (1 << 21)
         out = {
             "metric": METRIC if width == 8 else "Mrays/s primary closest-hit", "value": round(value, 3),
             "unit": UNIT, "n_gpus": world, "steps": args.steps,
@@ -385,10 +384,7 @@ def run_ours(args):
                  if args.builder in MORTON_TREES else {})) | (
                 {"parallelism": f"replicas x{world}", "build_seconds": round(info["build_seconds"], 2),
                  "tree_device_bytes": info["device_bytes"],
-                 "schedule": "rays in the order of a 30-bit coherence key (hand-written stable radix sort, "
-                             "3 passes of 10 bits), then one per thread (default for >= 2^21 closest-hit rays; the "
-                             "sort is inside the timed step)"
-                             if sorted_schedule else "one ray per thread"}),
+                 "schedule": "batch order, a ray per lane, leaves tested by eight lanes, idle lanes refilled"}),
             "roofline": {"bound": bound, "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
                          "frac": round(achieved / peak, 4), "traffic": traffic,
                          "peak_source": peak_src,
@@ -403,10 +399,7 @@ def run_ours(args):
             "e2e": {"value": round(e2e_value, 3), "unit": UNIT, "h2d_bytes_per_step": int(n * 32),
                     "d2h_bytes_per_step": int(n * 16)},
             "clocks": clocks.summary(),
-            # the default schedule sorts closest-hit batches of >= 2^21 FP32 rays: the key kernel (which also
-            # counts the first digit), then per 10-bit digit a tile scan, a tile-sum scan and a scatter, the
-            # next digit's count between passes, then the traversal kernel: 13 launches for 4M rays
-            "gpu_launches": args.steps * (13 if sorted_schedule else 1),
+            "gpu_launches": args.steps,  # one traversal launch per step
             **({"parity_vs_fp32_nodes": parity} if parity else {}),
         }
         if world == 1 and not args.no_cpu_baseline:

@@ -166,8 +166,8 @@ typedef enum {
                                        direction) so that concurrent warps read the same nodes; batches of
                                        65,536 rays or more; scratch (16 B per ray) from a stream-ordered
                                        pool */
-    SG_SCHEDULE_AUTO = 5            /* a new scene's default: SORTED for closest-hit batches of 2M rays or
-                                       more, THREAD_PER_RAY otherwise */
+    SG_SCHEDULE_AUTO = 5            /* a new scene's default: the faster one, THREAD_PER_RAY (sorting costs
+                                       more than it saves, also on rays in random order) */
 } sg_schedule;
 
 typedef struct {

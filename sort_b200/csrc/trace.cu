@@ -20,8 +20,8 @@
 // (sg_trace_stats) run Traversal, one ray per thread, whose node and triangle
 // visits are SORT's one by one. Schedules change the order in which rays are
 // taken, never a result: batch order, or the order of a coherence key (direction
-// octant, origin cell, coarse direction), which the automatic default uses for
-// large closest-hit batches so that concurrent warps read the same nodes.
+// octant, origin cell, coarse direction), so that concurrent warps read the same
+// nodes.
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -255,10 +255,9 @@ static cudaError_t launch_walk(const TraceLaunch& L, const DevTree& tr, const De
 }
 
 // ---------------------------------------------------------------------------
-// Sorted schedule (SG_SCHEDULE_SORTED, and the automatic choice for large
-// closest-hit batches): rays are put in the order of a 30-bit coherence key
-// before the thread-per-ray traversal, so that a warp holds rays that start
-// near one another and head the same way and take more of the same branches.
+// Sorted schedule (SG_SCHEDULE_SORTED): rays are taken in the order of a 30-bit
+// coherence key, so that the rays in traversal at one time start near one another
+// and head the same way.
 // The key: direction octant (3 bits), the Morton code of the origin's cell on a
 // 128^3 grid over the scene box (21 bits), then 2 bits per axis of direction.
 //
@@ -275,14 +274,8 @@ static cudaError_t launch_walk(const TraceLaunch& L, const DevTree& tr, const De
 //    into per-warp starting places, and each warp writes its keys in order
 //    (lanes of one digit ranked by __match_any_sync), which keeps the sort
 //    stable;
-//  * k_trace_walk with `order`: thread k traces ray order[k] and writes its
-//    answer at that ray's own index, so results do not depend on the order.
-// Measured on 4,194,304 incoherent rays (21M triangles): 1,034.5 Mrays/s
-// including the sort, against 1,031.1 with CUB's radix sort of the same keys
-// (same order) and 968.7 unsorted. Sorting only the key's top 10 or 20 bits
-// (one or two passes, batch order inside each group) gave 936 and 974, and
-// single-pass bucketing whose order inside a bucket followed warp timing gave
-// 902-954: the order inside a group matters.
+//  * k_trace_walk with `order`: the k-th ray taken is ray order[k], and its
+//    answer goes to that ray's own index, so results do not depend on the order.
 constexpr int kKeyBits = 30;
 constexpr int kSortBits = 30;  // top bits of the key that are sorted
 using psort::kDigits;
@@ -391,13 +384,13 @@ static cudaError_t launch_stack(const TraceLaunch& L, const DevTree& tr, const D
                                                                        L.stats, L.n_dev);
         return cudaGetLastError();
     }
-    // Batches large enough for reordering to pay; the automatic choice sorts
-    // large closest-hit batches only (any-hit rays end early, and measured no
-    // faster sorted).
-    const bool sorted = L.tuning.schedule == kScheduleSorted ? n >= (int64_t(1) << 16)
-                        : L.tuning.schedule == kScheduleAuto  ? !ANY && n >= (int64_t(1) << 21)
-                                                              : false;
-    if (!L.n_dev && sorted && n <= kMaxWalkRays)
+    // The automatic choice is batch order at every size: with lanes refilled and
+    // leaves shared, a warp's rays need not be alike, and the sort costs more than
+    // the cache lines it saves. Batch order against sorted, ms, 21M triangles, 4M
+    // rays (1M rays): diffuse 2.19 / 2.50 (0.61 / 0.73), shuffled at random 2.52 /
+    // 2.69 (0.70 / 0.80); camera 1.58 / 1.79, shuffled 2.33 / 2.50; shadow 2.09 /
+    // 2.26, shuffled 2.44 / 2.50.
+    if (L.tuning.schedule == kScheduleSorted && !L.n_dev && n >= (int64_t(1) << 16) && n <= kMaxWalkRays)
         return L.q8 ? launch_sorted<W, ANY, STACK, true>(L, tr, rays, n, s)
                     : launch_sorted<W, ANY, STACK, false>(L, tr, rays, n, s);
     return L.q8 ? launch_walk<W, ANY, STACK, true>(L, tr, rays, n, nullptr, L.counter, s)

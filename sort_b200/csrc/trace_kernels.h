@@ -14,7 +14,7 @@ constexpr int kSchedulePersistent = 1;    // the same, refilling at tuning.refil
 constexpr int kScheduleWhileWhile = 2;    // as 0
 constexpr int kScheduleSpeculative = 3;   // as 0
 constexpr int kScheduleSorted = 4;        // rays taken in the order of a coherence key
-constexpr int kScheduleAuto = 5;          // sorted for large closest-hit batches, else batch order
+constexpr int kScheduleAuto = 5;          // batch order
 
 struct TraceTuning {
     int schedule = kScheduleAuto;
