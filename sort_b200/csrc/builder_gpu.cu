@@ -23,13 +23,16 @@
 //     k-th element of the left part that fails the predicate is swapped with
 //     the k-th element from the right end of the right part that passes it,
 //     so the result is found with two prefix sums and one swap per pair.
+// Nodes of at most kSmall primitives leave the rounds: one warp splits such a
+// node whole, level by level (k_split_small).
 // Centroids and primitive boxes travel with the primitives (slot order), so
 // every pass reads them coalesced. The nodes under construction live on the
 // GPU too, in primitive-range order: after the passes, one thread per node
 // applies its split to the node's range lists, a finished node writes its
 // children as shape nodes, and prefix sums place the continuing nodes and the
 // new ones in the next round's list. A round costs one 16-byte download (the
-// sizes of the next round). The host only flattens the finished shape tree.
+// sizes of the next round). The nodes are numbered on the device; the host
+// flattens the finished shape tree only where a scene keeps host arrays.
 // The tree, the leaf order and every box value are build_tree's; a box bound
 // that is zero may carry the other sign, which no comparison sees.
 #include <cuda_runtime.h>
@@ -132,6 +135,7 @@ struct BuildState {
     int rounds;     // rounds that split something
     int next;       // this round's results, consumed by k_advance
     int new_shapes;
+    int small[2];   // small nodes waiting (k_split_small): this pass's and the next one's
 };
 
 __device__ __forceinline__ int find_range(const int64_t* __restrict__ starts, const int64_t* __restrict__ ends,
@@ -461,17 +465,32 @@ struct DNode {
     DRange done[8];
 };
 
-// The tree before flattening: a node's children are consecutive shape ids.
+// The tree before flattening: a node's children are consecutive shape ids,
+// above their parent's.
 struct DShape {
     int32_t off, cnt, first_kid, nkids;
+    int32_t depth;
     float mn[3], mx[3];  // box of the primitive range (the parent's child box)
+};
+
+// A node of at most kSmall primitives, split by one warp (k_split_small).
+// Large nodes go through the rounds, whose passes over every primitive cost the
+// same however few are still being split: without small nodes a 5.2M-triangle
+// tree took 72 rounds of 0.45 ms, most of them for ranges of a few hundred.
+constexpr int kSmall = 1024;
+struct SmallNode {
+    int32_t id, depth;
+    DRange x;
 };
 
 __device__ __forceinline__ bool starts_node(const DRange& x, int depth, int max_leaf, int max_depth) {
     return (x.e - x.s) > max_leaf && depth != max_depth;  // else splitNode returns at once
 }
 
-__device__ __forceinline__ DRange make_range(int32_t s, int32_t e, const int (&img)[6]) {
+// Whether such a range goes to the rounds (and not to k_split_small).
+__device__ __forceinline__ bool is_large(const DRange& x) { return x.e - x.s > kSmall; }
+
+__device__ __forceinline__ DRange make_range(int32_t s, int32_t e, const int* img) {
     DRange x;
     x.s = s;
     x.e = e;
@@ -538,13 +557,13 @@ __global__ void k_node_apply(BuildState* __restrict__ bs, DNode* __restrict__ no
         int kid_max = 0;
         for (int q = head; q < tail; ++q) {
             if (starts_node(nd.fifo[q & 7], nd.depth + 1, max_leaf, max_depth))
-                ++next;
+                next += is_large(nd.fifo[q & 7]) ? 1 : 0;
             else
                 kid_max = nd.depth + 1;
         }
         for (int q = 0; q < ndone; ++q) {
             if (starts_node(nd.done[q], nd.depth + 1, max_leaf, max_depth))
-                ++next;
+                next += is_large(nd.done[q]) ? 1 : 0;
             else
                 kid_max = nd.depth + 1;
         }
@@ -564,11 +583,13 @@ __global__ void k_summary(BuildState* __restrict__ bs, const int* __restrict__ c
 
 // Finished nodes write their children (SORT's child order: the remaining list,
 // then the done list) as shape nodes; the next round's nodes are the
-// continuing ones and the new children, in primitive-range order.
-__global__ void k_node_commit(const BuildState* __restrict__ bs, const DNode* __restrict__ cur,
+// continuing ones and the new large children, in primitive-range order; the new
+// small children wait for k_split_small (in any order).
+__global__ void k_node_commit(BuildState* __restrict__ bs, const DNode* __restrict__ cur,
                               const int* __restrict__ off_next, const int* __restrict__ off_shape,
                               const int* __restrict__ cnt_shape, int W, int max_leaf, int max_depth,
-                              DShape* __restrict__ shapes, DNode* __restrict__ next) {
+                              DShape* __restrict__ shapes, DNode* __restrict__ next,
+                              SmallNode* __restrict__ small) {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= bs->na) return;
     const DNode& nd = cur[r];
@@ -594,6 +615,7 @@ __global__ void k_node_commit(const BuildState* __restrict__ bs, const DNode* __
         sh.cnt = ks[q].e - ks[q].s;
         sh.first_kid = -1;
         sh.nkids = 0;
+        sh.depth = nd.depth + 1;
         for (int a = 0; a < 3; ++a) {
             sh.mn[a] = ks[q].mn[a];
             sh.mx[a] = ks[q].mx[a];
@@ -609,6 +631,10 @@ __global__ void k_node_commit(const BuildState* __restrict__ bs, const DNode* __
     for (int j = 0; j < m; ++j) {
         const DRange& x = ks[ord[j]];
         if (!starts_node(x, depth, max_leaf, max_depth)) continue;
+        if (!is_large(x)) {
+            small[atomicAdd(&bs->small[0], 1)] = SmallNode{first + ord[j], depth, x};
+            continue;
+        }
         DNode& c = next[o++];
         c.id = first + ord[j];
         c.depth = depth;
@@ -617,6 +643,286 @@ __global__ void k_node_commit(const BuildState* __restrict__ bs, const DNode* __
         c.tail = 1;
         c.ndone = 0;
         c.fifo[0] = x;
+    }
+}
+
+// Splits small nodes, one warp per node, a node's whole W-way split at once:
+// the passes of a round (centroid bounds, bins, sweep, halves, partition) over
+// the node's own primitives, with the same arithmetic and the same order of
+// swaps. Its children that are nodes go to the next pass's list. One pass per
+// tree level; a warp reads its primitives from L1 and L2, so a pass is bound by
+// its instructions and shared-memory atomics, not by HBM.
+struct SmallShared {
+    unsigned cnt[kBins];
+    int box[kBins][6];
+    DRange fifo[8], done[8];
+};
+constexpr int kSmallWarps = 4;
+
+__device__ __forceinline__ void warp_box(int (&v)[6]) {
+    for (int a = 0; a < 3; ++a) {
+        v[a] = __reduce_min_sync(0xffffffffu, v[a]);
+        v[3 + a] = __reduce_max_sync(0xffffffffu, v[3 + a]);
+    }
+}
+
+// The split of range x (more than max_leaf primitives) of a node: the axis and
+// position pick_best_split finds, whether splitNode takes it (whole warp).
+__device__ __forceinline__ bool small_split(const DRange& x, float node_area, int64_t n, float* cx, float* cy, float* cz,
+                                            float* pb, SmallShared& sh, int lane, int& axis, float& split_pos) {
+    int v[6];
+    empty_box(v);
+    for (int i = x.s + lane; i < x.e; i += 32) {
+        const int c[3] = {f2o(cx[i]), f2o(cy[i]), f2o(cz[i])};
+        for (int a = 0; a < 3; ++a) {
+            v[a] = min(v[a], c[a]);
+            v[3 + a] = max(v[3 + a], c[a]);
+        }
+    }
+    warp_box(v);
+    RangeTask t;  // only its centroid bounds are used
+    for (int a = 0; a < 6; ++a) t.inner[a] = v[a];
+    float start, delta, inv;
+    if (!bin_geometry(t, axis, start, delta, inv)) return false;
+    if (lane < kBins) {
+        sh.cnt[lane] = 0;
+        empty_box(sh.box[lane]);
+    }
+    __syncwarp();
+    const float* c = axis == 0 ? cx : (axis == 1 ? cy : cz);
+    for (int i = x.s + lane; i < x.e; i += 32) {
+        int b = __float2int_rz(__fmul_rn(__fsub_rn(c[i], start), inv));
+        b = max(0, min(b, kBins - 1));
+        atomicAdd(&sh.cnt[b], 1u);
+        for (int a = 0; a < 3; ++a) {
+            atomicMin(&sh.box[b][a], f2o(pb[a * n + i]));
+            atomicMax(&sh.box[b][3 + a], f2o(pb[(3 + a) * n + i]));
+        }
+    }
+    __syncwarp();
+    // Lane i < 15: the cut after bin i. Boxes left and right of it are unions of
+    // bins (exact in any order), found by scans over the lanes; the positions
+    // accumulate one by one, as pick_best_split adds them.
+    unsigned left = lane < kBins ? sh.cnt[lane] : 0u;
+    int l[6], r[6];
+    empty_box(l);
+    if (lane < kBins)
+        for (int a = 0; a < 6; ++a) l[a] = sh.box[lane][a];
+    for (int a = 0; a < 6; ++a) r[a] = l[a];
+    for (int o = 1; o < kBins; o <<= 1) {
+        const unsigned pc = __shfl_up_sync(0xffffffffu, left, o);
+        int pl[6], pr[6];
+        for (int a = 0; a < 6; ++a) {
+            pl[a] = __shfl_up_sync(0xffffffffu, l[a], o);
+            pr[a] = __shfl_down_sync(0xffffffffu, r[a], o);  // lanes past the bins hold empty boxes
+        }
+        if (lane >= o) {
+            left += pc;
+            for (int a = 0; a < 3; ++a) {
+                l[a] = min(l[a], pl[a]);
+                l[3 + a] = max(l[3 + a], pl[3 + a]);
+            }
+        }
+        if (lane + o < kBins)
+            for (int a = 0; a < 3; ++a) {
+                r[a] = min(r[a], pr[a]);
+                r[3 + a] = max(r[3 + a], pr[3 + a]);
+            }
+    }
+    for (int a = 0; a < 6; ++a) r[a] = __shfl_down_sync(0xffffffffu, r[a], 1);  // bins i + 1 .. 15
+    float pos = __fadd_rn(delta, start), mine = pos;
+    for (int i = 1; i < kBins - 1; ++i) {
+        pos = __fadd_rn(pos, delta);
+        if (i == lane) mine = pos;
+    }
+    const unsigned total = (unsigned)(x.e - x.s);
+    float sah = FLT_MAX;
+    if (lane < kBins - 1) {
+        float lmn[3], lmx[3], rmn[3], rmx[3];
+        for (int a = 0; a < 3; ++a) {
+            lmn[a] = o2f(l[a]);
+            lmx[a] = o2f(l[3 + a]);
+            rmn[a] = o2f(r[a]);
+            rmx[a] = o2f(r[3 + a]);
+        }
+        const float ls = __fmul_rn(__uint2float_rn(left), half_area(lmn, lmx));
+        const float rs = __fmul_rn(__uint2float_rn(total - left), half_area(rmn, rmx));
+        sah = __fdiv_rn(__fadd_rn(ls, rs), node_area);
+    }
+    // The first cut of least cost (only costs below FLT_MAX count; NaN does not).
+    const bool valid = sah < FLT_MAX;
+    const int key = valid ? f2o(sah == 0.0f ? 0.0f : sah) : 0x7fffffff;
+    const int least = __reduce_min_sync(0xffffffffu, key);
+    const unsigned at = __ballot_sync(0xffffffffu, valid && key == least);
+    if (at == 0) return false;  // no cut below FLT_MAX: at least as dear as a leaf
+    const int best = __ffs(at) - 1;
+    split_pos = __shfl_sync(0xffffffffu, mine, best);
+    return !(__shfl_sync(0xffffffffu, sah, best) >= __uint2float_rn(total));
+}
+
+__global__ void __launch_bounds__(32 * kSmallWarps) k_split_small(
+    int64_t n, BuildState* __restrict__ bs, int in, const SmallNode* __restrict__ nodes, SmallNode* __restrict__ out,
+    int W, int max_leaf, int max_depth, float* cx, float* cy, float* cz, float* pb, int32_t* idx, int32_t* pl,
+    int32_t* pr, DShape* __restrict__ shapes) {
+    __shared__ SmallShared shared[kSmallWarps];
+    SmallShared& sh = shared[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const int count = bs->small[in], stride = (int)gridDim.x * kSmallWarps;
+    for (int w = (int)blockIdx.x * kSmallWarps + (threadIdx.x >> 5); w < count; w += stride) {
+        const SmallNode nd = nodes[w];
+        const float area = half_area(nd.x.mn, nd.x.mx);
+        int head = 0, tail = 1, ndone = 0;
+        __syncwarp();
+        if (lane == 0) sh.fifo[0] = nd.x;
+        __syncwarp();
+        // SORT's loop: the front range is split or set aside until the list is
+        // empty or the node has W ranges.
+        do {
+            const DRange x = sh.fifo[head++ & 7];
+            int axis = 0;
+            float pos = 0.0f;
+            int mid = x.s;
+            int lb[6], rb[6];
+            if (x.e - x.s > max_leaf && small_split(x, area, n, cx, cy, cz, pb, sh, lane, axis, pos)) {
+                // Both halves' sizes and primitive boxes.
+                const float* c = axis == 0 ? cx : (axis == 1 ? cy : cz);
+                int pass = 0;
+                empty_box(lb);
+                empty_box(rb);
+                for (int i = x.s + lane; i < x.e; i += 32) {
+                    const bool p = c[i] < pos;
+                    pass += p ? 1 : 0;
+                    for (int a = 0; a < 3; ++a) {
+                        const int lo = f2o(pb[a * n + i]), hi = f2o(pb[(3 + a) * n + i]);
+                        if (p) {
+                            lb[a] = min(lb[a], lo);
+                            lb[3 + a] = max(lb[3 + a], hi);
+                        } else {
+                            rb[a] = min(rb[a], lo);
+                            rb[3 + a] = max(rb[3 + a], hi);
+                        }
+                    }
+                }
+                mid = x.s + (int)__reduce_add_sync(0xffffffffu, (unsigned)pass);
+                warp_box(lb);
+                warp_box(rb);
+                if (mid != x.s && mid != x.e) {
+                    // std::partition: the k-th failing element left of mid is
+                    // swapped with the k-th passing one from the right end.
+                    int nl = 0, nr = 0;
+                    for (int b = x.s; b < mid; b += 32) {
+                        const int i = b + lane;
+                        const bool m = i < mid && !(c[i] < pos);
+                        const unsigned bal = __ballot_sync(0xffffffffu, m);
+                        if (m) pl[x.s + nl + __popc(bal & below)] = i;
+                        nl += __popc(bal);
+                    }
+                    for (int b = x.e - 1; b >= mid; b -= 32) {
+                        const int i = b - lane;
+                        const bool m = i >= mid && c[i] < pos;
+                        const unsigned bal = __ballot_sync(0xffffffffu, m);
+                        if (m) pr[x.s + nr + __popc(bal & below)] = i;
+                        nr += __popc(bal);
+                    }
+                    __syncwarp();
+                    for (int k = lane; k < nl; k += 32) {
+                        const int64_t i = pl[x.s + k], j = pr[x.s + k];
+                        swap_at(cx, i, j);
+                        swap_at(cy, i, j);
+                        swap_at(cz, i, j);
+                        swap_at(idx, i, j);
+                        for (int q = 0; q < 6; ++q) swap_at(pb + q * n, i, j);
+                    }
+                }
+            }
+            __syncwarp();
+            if (mid == x.s || mid == x.e) {
+                if (lane == 0) sh.done[ndone] = x;
+                ++ndone;
+            } else {
+                if (lane == 0) {
+                    sh.fifo[tail & 7] = make_range(x.s, mid, lb);
+                    sh.fifo[(tail + 1) & 7] = make_range(mid, x.e, rb);
+                }
+                tail += 2;
+            }
+            __syncwarp();
+        } while (head != tail && (tail - head) + ndone < W);
+        const int total = (tail - head) + ndone;
+        if (total == 1) {  // a single range: the node is a leaf
+            if (lane == 0) atomicMax(&bs->depth_max, nd.depth);
+            continue;
+        }
+        int first = 0;
+        if (lane == 0) {
+            first = atomicAdd(&bs->shapes, total);
+            shapes[nd.id].first_kid = first;
+            shapes[nd.id].nkids = total;
+        }
+        first = __shfl_sync(0xffffffffu, first, 0);
+        if (lane < total) {
+            const int rest = tail - head;
+            const DRange x = lane < rest ? sh.fifo[(head + lane) & 7] : sh.done[lane - rest];
+            DShape& k = shapes[first + lane];
+            k.off = x.s;
+            k.cnt = x.e - x.s;
+            k.first_kid = -1;
+            k.nkids = 0;
+            k.depth = nd.depth + 1;
+            for (int a = 0; a < 3; ++a) {
+                k.mn[a] = x.mn[a];
+                k.mx[a] = x.mx[a];
+            }
+            if (starts_node(x, nd.depth + 1, max_leaf, max_depth))
+                out[atomicAdd(&bs->small[in ^ 1], 1)] = SmallNode{first + lane, nd.depth + 1, x};
+            else
+                atomicMax(&bs->depth_max, nd.depth + 1);
+        }
+    }
+}
+
+// The lists change places after a pass.
+__global__ void k_small_next(BuildState* __restrict__ bs, int in) { bs->small[in] = 0; }
+
+// ---- Node numbering on the device --------------------------------------------
+// build_tree's numbers: a node's interior children get consecutive numbers when
+// it is filled, and nodes are filled depth-first, first child first. With
+// inner[c] the interior nodes strictly below shape c, a node whose children
+// start at base numbers them base .. base + k - 1, and child j's own children
+// start at base + k + the sum of inner over the interior children before it.
+// One pass per level, bottom-up for inner, top-down for the numbers.
+__global__ void k_count_inner(int count, int depth, const DShape* __restrict__ shapes, int32_t* __restrict__ inner) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count || shapes[i].depth != depth) return;
+    int sum = 0;
+    const int k = shapes[i].nkids, f = shapes[i].first_kid;
+    for (int j = 0; j < k; ++j)
+        if (shapes[f + j].nkids) sum += 1 + inner[f + j];
+    inner[i] = sum;
+}
+
+__global__ void k_number(int count, int depth, const DShape* __restrict__ shapes, const int32_t* __restrict__ inner,
+                         int32_t* __restrict__ number, int32_t* __restrict__ base_of, int32_t* __restrict__ node_shape,
+                         int32_t* __restrict__ node_base) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count || shapes[i].depth != depth || shapes[i].nkids == 0) return;
+    const int k = shapes[i].nkids, f = shapes[i].first_kid;
+    if (i == 0) {  // the root
+        number[0] = 0;
+        base_of[0] = 1;
+    }
+    const int base = base_of[i];
+    node_shape[number[i]] = i;
+    node_base[number[i]] = base;
+    int interior = 0, at = 0;
+    for (int j = 0; j < k; ++j) interior += shapes[f + j].nkids ? 1 : 0;
+    int below = base + interior;
+    for (int j = 0; j < k; ++j) {
+        if (shapes[f + j].nkids == 0) continue;
+        number[f + j] = base + at++;
+        base_of[f + j] = below;
+        below += inner[f + j];
     }
 }
 
@@ -765,8 +1071,13 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
     if (n == 0) return t;
 
     // Node-sized buffers at their bounds: nodes under construction own disjoint
-    // ranges of more than max_leaf primitives; the tree has fewer than 2n nodes.
-    const int64_t cap = std::min<int64_t>(n, n / (int64_t(p.max_leaf) + 1) + 1);
+    // ranges of more than max_leaf primitives, the rounds' of more than kSmall;
+    // the tree has fewer than 2n nodes.
+    const int64_t small_cap = std::min<int64_t>(n, n / (int64_t(p.max_leaf) + 1) + 1);
+    const int64_t cap = std::min<int64_t>(small_cap, n / (int64_t(kSmall) + 1) + 1);
+    DevBuf<SmallNode> d_small, d_small_next;
+    d_small.alloc(size_t(small_cap));
+    d_small_next.alloc(size_t(small_cap));
     d_cur.alloc(size_t(cap));
     d_next.alloc(size_t(cap));
     d_rt.alloc(size_t(cap));
@@ -794,22 +1105,28 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
 
     // The root shape, and the root node unless splitNode returns at once.
     {
-        DShape root{0, int32_t(n), -1, 0, {scene.mn[0], scene.mn[1], scene.mn[2]},
+        DShape root{0, int32_t(n), -1, 0, 1, {scene.mn[0], scene.mn[1], scene.mn[2]},
                     {scene.mx[0], scene.mx[1], scene.mx[2]}};
         check(cudaMemcpyAsync(d_shapes.p, &root, sizeof(root), cudaMemcpyHostToDevice, st), "root");
     }
     const bool root_node = n > p.max_leaf && p.max_depth != 1;
-    *h_state.p = BuildState{root_node ? 1 : 0, 1, root_node ? 0 : 1, 0, 0, 0};
+    const bool large_root = root_node && n > kSmall, small_root = root_node && !large_root;
+    *h_state.p = BuildState{large_root ? 1 : 0, 1, root_node ? 0 : 1, 0, 0, 0, {small_root ? 1 : 0, 0}};
     check(cudaMemcpyAsync(d_state.p, h_state.p, sizeof(BuildState), cudaMemcpyHostToDevice, st), "state");
+    DNode root{};
+    SmallNode root_small{};
     if (root_node) {
-        DNode root{};
         root.id = 0;
         root.depth = 1;
         root.area = host_half_area(scene);
         root.tail = 1;
         root.fifo[0] = DRange{0, int32_t(n), {scene.mn[0], scene.mn[1], scene.mn[2]},
                               {scene.mx[0], scene.mx[1], scene.mx[2]}};
-        check(cudaMemcpyAsync(d_cur.p, &root, sizeof(root), cudaMemcpyHostToDevice, st), "root");
+        root_small = SmallNode{0, 1, root.fifo[0]};
+        if (large_root)
+            check(cudaMemcpyAsync(d_cur.p, &root, sizeof(root), cudaMemcpyHostToDevice, st), "root");
+        else
+            check(cudaMemcpyAsync(d_small.p, &root_small, sizeof(root_small), cudaMemcpyHostToDevice, st), "root");
     }
     check(cudaStreamSynchronize(st), "root");
 
@@ -821,7 +1138,7 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
     const int64_t max_rounds = int64_t(W - 1) * p.max_depth + 1;
     const unsigned ng = grid(cap, 128);
     int64_t queued = 0;
-    while (root_node) {
+    while (large_root) {
         for (int g = 0; g < kGroup; ++g) {
             k_node_ranges<<<ng, 128, 0, st>>>(d_state.p, d_cur.p, d_rt.p, d_starts.p, d_ends.p);
             k_bounds<<<grid(n), 256, 0, st>>>(n, d_starts.p, d_ends.p, d_state.p, d_cx.p, d_cy.p, d_cz.p, d_rid.p,
@@ -843,7 +1160,7 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
             scan(d_cnt_shape.p, d_off_shape.p, cap);
             k_summary<<<1, 1, 0, st>>>(d_state.p, d_cnt_next.p, d_off_next.p, d_cnt_shape.p, d_off_shape.p);
             k_node_commit<<<ng, 128, 0, st>>>(d_state.p, d_cur.p, d_off_next.p, d_off_shape.p, d_cnt_shape.p, W,
-                                              p.max_leaf, p.max_depth, d_shapes.p, d_next.p);
+                                              p.max_leaf, p.max_depth, d_shapes.p, d_next.p, d_small.p);
             k_advance<<<1, 1, 0, st>>>(d_state.p);
             check(cudaGetLastError(), "node commit");
             swap_bufs(d_cur, d_next);
@@ -854,106 +1171,148 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
         if (h_state.p->na == 0) break;
         if (queued > max_rounds) throw std::runtime_error("GPU build: the split rounds did not finish");
     }
+    // The small nodes, one pass per level of the tree (a node's children are one
+    // level below it, and the depth is capped).
+    int passes = 0;
+    if (root_node) {
+        int32_t* pl32 = reinterpret_cast<int32_t*>(d_pl.p);  // the rounds are done with the pair lists
+        int32_t* pr32 = reinterpret_cast<int32_t*>(d_pr.p);
+        int in = 0;
+        for (;;) {
+            const int count = h_state.p->small[in];
+            if (count == 0) break;
+            if (++passes > p.max_depth) throw std::runtime_error("GPU build: the small splits did not finish");
+            k_split_small<<<std::min<unsigned>(grid(count, kSmallWarps), 148 * 16), 32 * kSmallWarps, 0, st>>>(
+                n, d_state.p, in, d_small.p, d_small_next.p, W, p.max_leaf, p.max_depth, d_cx.p, d_cy.p, d_cz.p,
+                d_pb.p, d_idx.p, pl32, pr32, d_shapes.p);
+            k_small_next<<<1, 1, 0, st>>>(d_state.p, in);
+            check(cudaGetLastError(), "small splits");
+            swap_bufs(d_small, d_small_next);
+            in ^= 1;
+            check(cudaMemcpyAsync(h_state.p, d_state.p, sizeof(BuildState), cudaMemcpyDeviceToHost, st), "state");
+            check(cudaStreamSynchronize(st), "small splits");
+        }
+    }
     const BuildState fin = *h_state.p;
     const int shape_count = fin.shapes;
     t.depth = fin.depth_max;
 
-    // Shapes and the final permutation (leaf order) to the host, through the
-    // device's pinned staging memory (pageable copies of these 130 MB cost
-    // about 100 ms).
-    Staging& stage = staging(device);
-    std::lock_guard<std::mutex> stage_lock(stage.lock);
     // Host arrays (child references, leaf order and flags) only where the scene
     // reads them: 8-bit nodes and mixed primitives. A triangle scene with FP32
     // nodes takes its nodes and records from the device (its topology export
     // reads them back from there).
     const bool host = p.host_boxes || p.nextra > 0;
-    const size_t shape_bytes = (size_t(shape_count) * sizeof(DShape) + 255) & ~size_t(255);
-    const size_t stage_bytes = shape_bytes + (host ? size_t(n) * 4 : 0);
-    if (stage.bytes < stage_bytes) {
-        if (stage.p) cudaFreeHost(stage.p);
-        stage.p = nullptr;
-        stage.bytes = 0;
-        check(cudaMallocHost(&stage.p, stage_bytes), "cudaMallocHost(staging)");
-        stage.bytes = stage_bytes;
-    }
-    const DShape* shape = static_cast<const DShape*>(stage.p);
-    const int32_t* h_order = reinterpret_cast<const int32_t*>(static_cast<const char*>(stage.p) + shape_bytes);
-    check(cudaMemcpyAsync(stage.p, d_shapes.p, size_t(shape_count) * sizeof(DShape), cudaMemcpyDeviceToHost, st),
-          "shapes");
-    if (host)
-        check(cudaMemcpyAsync(const_cast<int32_t*>(h_order), d_idx.p, size_t(n) * 4, cudaMemcpyDeviceToHost, st),
-              "order");
-    check(cudaStreamSynchronize(st), "download");
-    if (host) {
-        t.order.assign(h_order, h_order + n);
-        t.leaf_last.assign(size_t(n), 0);
-    }
-    // Flatten exactly as build_tree numbers nodes: a node allocates its interior
-    // children consecutively when it is filled, then fills them in order. The
-    // arrays are sized once (the interior count is known), then filled.
+    // The nodes' numbers (build_tree's, see k_count_inner): on the host this took
+    // 10 ms for 5.2M triangles beside 2 ms of copies.
+    DevBuf<int32_t> d_inner, d_number, d_base, d_map;
     size_t interior_total = 0;
-    for (int s_ = 0; s_ < shape_count; ++s_) interior_total += shape[s_].nkids ? 1 : 0;
-    if (host) {
-        t.first_interior.assign(interior_total, -1);
-        t.child.assign(interior_total * W, kEmptyRef);
-    } else {
+    if (root_node) {
+        d_inner.alloc(size_t(shape_count));
+        d_number.alloc(size_t(shape_count));
+        d_base.alloc(size_t(shape_count));
+        for (int d = t.depth; d >= 1; --d)
+            k_count_inner<<<grid(shape_count), 256, 0, st>>>(shape_count, d, d_shapes.p, d_inner.p);
+        check(cudaGetLastError(), "node numbers");
+        int32_t below = 0;
+        DShape top;
+        check(cudaMemcpyAsync(&below, d_inner.p, 4, cudaMemcpyDeviceToHost, st), "node numbers");
+        check(cudaMemcpyAsync(&top, d_shapes.p, sizeof(top), cudaMemcpyDeviceToHost, st), "node numbers");
+        check(cudaStreamSynchronize(st), "node numbers");
+        interior_total = top.nkids ? size_t(below) + 1 : 0;
+        if (interior_total > 0) {
+            d_map.alloc(2 * interior_total);
+            for (int d = 1; d <= t.depth; ++d)
+                k_number<<<grid(shape_count), 256, 0, st>>>(shape_count, d, d_shapes.p, d_inner.p, d_number.p,
+                                                           d_base.p, d_map.p, d_map.p + interior_total);
+            check(cudaGetLastError(), "node numbers");
+        }
+    }
+    if (!host) {
         t.n_interior = int64_t(interior_total);
         t.n_tri = n;
+        t.root = interior_total > 0 ? 0 : leaf_ref(0);
+        t.leaves = int64_t(shape_count) - int64_t(interior_total);
     }
-    if (p.host_boxes) {  // only a scene with 8-bit nodes reads the boxes on the host
-        t.lo.assign(interior_total * 3 * W, FLT_MAX);
-        t.hi.assign(interior_total * 3 * W, -FLT_MAX);
-    }
-    std::vector<int32_t> shape_of(interior_total);  // the shape each interior node came from
-    std::vector<int32_t> base_of(interior_total);   // and its first interior child
-    int32_t allocated = 0;
-    auto leaf = [&](const DShape& sn) {
-        t.leaves++;
-        if (host) t.leaf_last[size_t(sn.off + sn.cnt - 1)] = 1;
-    };
-    std::vector<std::pair<int, int32_t>> stack;  // (shape id, node index), filled depth-first in order
-    stack.reserve(64 * 8);
-    if (shape[0].nkids == 0) {
-        t.root = leaf_ref(0);
-        leaf(shape[0]);
-    } else {
-        t.root = allocated++;
-        stack.push_back({0, t.root});
-    }
-    while (!stack.empty()) {
-        const auto [sid, idx] = stack.back();
-        stack.pop_back();
-        const DShape& sn = shape[sid];
-        shape_of[size_t(idx)] = sid;
-        int interior = 0;
-        for (int j = 0; j < sn.nkids; ++j) interior += shape[sn.first_kid + j].nkids ? 1 : 0;
-        const int32_t base = interior ? allocated : -1;
-        allocated += interior;
-        base_of[size_t(idx)] = base;
-        if (host) t.first_interior[size_t(idx)] = base;
-        int k = 0;
-        std::pair<int, int32_t> sub[8];
-        int nsub = 0;
-        for (int j = 0; j < sn.nkids; ++j) {
-            const int kid_id = sn.first_kid + j;
-            const DShape& kid = shape[kid_id];
-            int32_t ref;
-            if (kid.nkids == 0) {
-                ref = leaf_ref(kid.off);
-                leaf(kid);
-            } else {
-                ref = base + k++;
-                sub[nsub++] = {kid_id, ref};
-            }
-            if (host) t.child[size_t(idx) * W + j] = ref;
-            if (p.host_boxes)
-                for (int a = 0; a < 3; ++a) {
-                    t.lo[(size_t(idx) * 3 + a) * W + j] = kid.mn[a];
-                    t.hi[(size_t(idx) * 3 + a) * W + j] = kid.mx[a];
-                }
+
+    if (host) {
+        // Shapes and the final permutation (leaf order) to the host, through the
+        // device's pinned staging memory (pageable copies of these 130 MB cost
+        // about 100 ms).
+        Staging& stage = staging(device);
+        std::lock_guard<std::mutex> stage_lock(stage.lock);
+        const size_t shape_bytes = (size_t(shape_count) * sizeof(DShape) + 255) & ~size_t(255);
+        const size_t stage_bytes = shape_bytes + size_t(n) * 4;
+        if (stage.bytes < stage_bytes) {
+            if (stage.p) cudaFreeHost(stage.p);
+            stage.p = nullptr;
+            stage.bytes = 0;
+            check(cudaMallocHost(&stage.p, stage_bytes), "cudaMallocHost(staging)");
+            stage.bytes = stage_bytes;
         }
-        for (int q = nsub - 1; q >= 0; --q) stack.push_back(sub[q]);  // first child filled next
+        const DShape* shape = static_cast<const DShape*>(stage.p);
+        const int32_t* h_order = reinterpret_cast<const int32_t*>(static_cast<const char*>(stage.p) + shape_bytes);
+        check(cudaMemcpyAsync(stage.p, d_shapes.p, size_t(shape_count) * sizeof(DShape), cudaMemcpyDeviceToHost, st),
+              "shapes");
+        check(cudaMemcpyAsync(const_cast<int32_t*>(h_order), d_idx.p, size_t(n) * 4, cudaMemcpyDeviceToHost, st),
+              "order");
+        check(cudaStreamSynchronize(st), "download");
+        t.order.assign(h_order, h_order + n);
+        t.leaf_last.assign(size_t(n), 0);
+        // Flatten exactly as build_tree numbers nodes: a node allocates its interior
+        // children consecutively when it is filled, then fills them in order. The
+        // arrays are sized once (the interior count is known), then filled.
+        t.first_interior.assign(interior_total, -1);
+        t.child.assign(interior_total * W, kEmptyRef);
+        if (p.host_boxes) {  // only a scene with 8-bit nodes reads the boxes on the host
+            t.lo.assign(interior_total * 3 * W, FLT_MAX);
+            t.hi.assign(interior_total * 3 * W, -FLT_MAX);
+        }
+        int32_t allocated = 0;
+        auto leaf = [&](const DShape& sn) {
+            t.leaves++;
+            t.leaf_last[size_t(sn.off + sn.cnt - 1)] = 1;
+        };
+        std::vector<std::pair<int, int32_t>> stack;  // (shape id, node index), filled depth-first in order
+        stack.reserve(64 * 8);
+        if (shape[0].nkids == 0) {
+            t.root = leaf_ref(0);
+            leaf(shape[0]);
+        } else {
+            t.root = allocated++;
+            stack.push_back({0, t.root});
+        }
+        while (!stack.empty()) {
+            const auto [sid, idx] = stack.back();
+            stack.pop_back();
+            const DShape& sn = shape[sid];
+            int interior = 0;
+            for (int j = 0; j < sn.nkids; ++j) interior += shape[sn.first_kid + j].nkids ? 1 : 0;
+            const int32_t base = interior ? allocated : -1;
+            allocated += interior;
+            t.first_interior[size_t(idx)] = base;
+            int k = 0;
+            std::pair<int, int32_t> sub[8];
+            int nsub = 0;
+            for (int j = 0; j < sn.nkids; ++j) {
+                const int kid_id = sn.first_kid + j;
+                const DShape& kid = shape[kid_id];
+                int32_t ref;
+                if (kid.nkids == 0) {
+                    ref = leaf_ref(kid.off);
+                    leaf(kid);
+                } else {
+                    ref = base + k++;
+                    sub[nsub++] = {kid_id, ref};
+                }
+                t.child[size_t(idx) * W + j] = ref;
+                if (p.host_boxes)
+                    for (int a = 0; a < 3; ++a) {
+                        t.lo[(size_t(idx) * 3 + a) * W + j] = kid.mn[a];
+                        t.hi[(size_t(idx) * 3 + a) * W + j] = kid.mx[a];
+                    }
+            }
+            for (int q = nsub - 1; q >= 0; --q) stack.push_back(sub[q]);  // first child filled next
+        }
     }
 
     // The interior nodes in the device layout, written where the shapes are
@@ -966,10 +1325,6 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
         }
     } nodes_owned;
     if (interior_total > 0) {
-        DevBuf<int32_t> d_map;
-        d_map.alloc(2 * interior_total);
-        check(upload_host(d_map.p, shape_of.data(), interior_total * 4, st), "node map");
-        check(upload_host(d_map.p + interior_total, base_of.data(), interior_total * 4, st), "node map");
         const int F4 = W == 8 ? NodeShape<8>::kF4 : NodeShape<4>::kF4;
         check(cudaMalloc(&nodes_owned.p, interior_total * F4 * sizeof(float4)), "cudaMalloc(nodes)");
         if (W == 8)
@@ -982,10 +1337,11 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
         check(cudaStreamSynchronize(st), "write nodes");
     }
 
-    // This file's kernels: setup and scene box, 13 per queued round, the node
-    // writer, the triangle records (the prefix sums are counted apart, four per round).
-    t.rounds = int(fin.rounds);
-    t.launches = int(4 + 13 * queued + (host ? 0 : 1));
+    // This file's kernels: setup and scene box, 13 per queued round, two per pass
+    // over the small nodes, two per level for the node numbers, the node writer,
+    // the triangle records (the prefix sums are counted apart, four per round).
+    t.rounds = int(fin.rounds) + passes;
+    t.launches = int(4 + 13 * queued + 2 * passes + (interior_total ? 2 * t.depth : 0) + (host ? 0 : 1));
     if (p.nextra > 0) {  // mixed primitives: the scene writes its slot records on the host
         t.d_nodes = nodes_owned.p;
         nodes_owned.p = nullptr;
