@@ -189,7 +189,8 @@ __global__ void __launch_bounds__(kWalkThreads, kSrvTraceBlocks)
     const int warps = (int)gridDim.x * kWalkWarps, share = (n + warps - 1) / warps;
     SrvJob job{scenes, ray,   scene_of, cap, first, n, prim, t, ANY ? occ : nullptr, taken,
                share < 32 ? (1u << share) - 1u : kFullWarp, false};
-    walk_rays<W, ANY, STACK, Q8, true>(job, &shared[threadIdx.x >> 5], (int)(threadIdx.x & 31u), 10, err);
+    walk_rays<W, ANY, STACK, Q8, true>(job, &shared[threadIdx.x >> 5], (int)(threadIdx.x & 31u), Q8 ? 12 : 24,
+                                       err);
 }
 
 __global__ void k_srv_shade(SrvBuffers b, const float* __restrict__ qray, const int* __restrict__ qslot,

@@ -76,12 +76,16 @@ __global__ void __launch_bounds__(128, 9) k_trace_stats(DevTree tr, DevRays rays
 // box, width 8: 7 blocks 2.54 / 2.10 ms on 4M diffuse / shadow rays (21M
 // triangles), 8 blocks (88 bytes spilled) 2.98 / 2.25, 9 blocks 2.96 / 2.40.
 // 8-bit nodes: 0.338 / 0.334 / 0.336 ms at 7 / 8 / 9 blocks on 700k rays.
-// Width 4, 1M camera rays: 0.207 / 0.207 / 0.201 ms at 7 / 8 / 9 blocks with a
-// refill at 10 idle lanes, 0.198 / 0.200 at 16 (4 idle lanes: 6% slower).
+// Width 4, 1M camera rays: 0.207 / 0.207 / 0.201 ms at 7 / 8 / 9 blocks.
+// Refills at 4 / 10 / 16 / 24 / 28 / 32 idle lanes: diffuse 2.40 / 2.19 / 2.20 /
+// 2.15 / 2.17 / 2.44 ms, shadow 2.29 / 2.09 / 2.09 / 2.05 / 2.05 / 2.13, camera
+// (width 4) 0.215 / 0.192 / 0.184 / 0.178 / 0.178 / 0.180; a refill is a ray's
+// setup at that many lanes, so it pays to wait. 8-bit nodes, whose visits cost
+// more, 0.336 / 0.325 / 0.328 / 0.340 / 0.351 / 0.398.
 template <int W, bool Q8>
 struct WalkShape {
     static constexpr int kBlocks = W == 8 && !Q8 ? 7 : 8;
-    static constexpr int kRefill = W == 8 ? 10 : 16;
+    static constexpr int kRefill = Q8 ? 12 : 24;
 };
 
 // Rays of a launch as its warps take them: one span of `span` rays per warp, or,
