@@ -171,7 +171,7 @@ BuiltTree build_tree_lbvh(const float* tri, int64_t ntri, const BuildParams& p, 
         check(cudaGetLastError(), "radix tree");
         launches += 2;
         levels = collapse_wide(t, bt, 0, W, p.max_leaf, d_perm.p, d_last.p, st);
-        launches += levels;
+        launches += levels + 1;
         perm = d_perm.p;
     }
     leaf_records(t, m.tri.p, n, perm, d_last.p, st);

@@ -242,7 +242,7 @@ BuiltTree build_tree_ploc(const float* tri, int64_t ntri, const BuildParams& p, 
         check(cudaStreamSynchronize(st), "root");
         const BinaryTree bt{d_left.p, d_right.p, d_count.p, d_ibox.p, m.sorted.p, m.pb.p, n};
         levels = collapse_wide(t, bt, root_rec.w, W, p.max_leaf, d_perm.p, d_last.p, st);
-        launches += levels;
+        launches += levels + 1;
         perm = d_perm.p;
     }
     leaf_records(t, m.tri.p, n, perm, d_last.p, st);

@@ -139,10 +139,25 @@ __device__ __forceinline__ float box_area(const float (&b)[6]) {
 }
 
 // The primitives under binary reference c, left to right, into slots
-// s .. s + k - 1 of perm: the k-th is found by descending from c with the
-// counts (each step shrinks the subtree, so at most k - 1 steps).
+// s .. s + k - 1 of perm: a depth-first walk whose stack holds the right
+// children still to visit (fewer than k); for a large leaf, whose walk would
+// not fit the stack, the r-th primitive by descending from c with the counts.
+constexpr int kLeafWalk = 16;
 __device__ __forceinline__ void leaf_slots(const BinaryTree& bt, int32_t c, int32_t s, int32_t k,
                                            int32_t* __restrict__ perm) {
+    if (k <= kLeafWalk) {
+        int32_t stack[kLeafWalk], node = c;
+        int sp = 0;
+        for (int32_t r = 0; r < k; ++r) {
+            while (node >= 0) {
+                stack[sp++] = bt.right[node];
+                node = bt.left[node];
+            }
+            perm[s + r] = bt.idx[~node];
+            if (sp > 0) node = stack[--sp];
+        }
+        return;
+    }
     for (int32_t r = 0; r < k; ++r) {
         int32_t node = c, rank = r;
         while (node >= 0) {
@@ -159,6 +174,19 @@ __device__ __forceinline__ void leaf_slots(const BinaryTree& bt, int32_t c, int3
     }
 }
 
+// Every leaf the collapse found (x: binary reference, y: first slot), one thread
+// each: within k_collapse a wide node's thread filled up to W leaves one after
+// another, a chain of dependent loads that set the length of every level.
+__global__ void k_fill_leaves(int count, const int2* __restrict__ leaves, BinaryTree bt, uint8_t* __restrict__ last,
+                              int32_t* __restrict__ perm) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const int2 leaf = leaves[i];
+    const int32_t k = ref_count(bt, leaf.x);
+    leaf_slots(bt, leaf.x, leaf.y, k, perm);
+    last[leaf.y + k - 1] = 1;
+}
+
 // One wide node per work item (x: binary node, y: wide index, z: first leaf
 // slot of the binary node's primitives). Children of at most max_leaf
 // primitives become leaves (free slots are first filled by opening such
@@ -166,8 +194,8 @@ __device__ __forceinline__ void leaf_slots(const BinaryTree& bt, int32_t c, int3
 // wide indices and go to the next level's queue at (index - next_base).
 template <int W>
 __global__ void k_collapse(int nq, const int4* __restrict__ q_in, int4* __restrict__ q_out, int next_base, int level,
-                           int max_leaf, BinaryTree bt, uint8_t* __restrict__ last, int32_t* __restrict__ perm,
-                           CollapseState* __restrict__ cs, float4* __restrict__ nodes) {
+                           int max_leaf, BinaryTree bt, int2* __restrict__ leaves, CollapseState* __restrict__ cs,
+                           float4* __restrict__ nodes) {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= nq) return;
     const int4 item = q_in[q];
@@ -179,17 +207,26 @@ __global__ void k_collapse(int nq, const int4* __restrict__ q_in, int4* __restri
     start[0] = item.z;
     start[1] = item.z + ref_count(bt, kid[0]);
     auto opens = [&](int32_t c) { return c >= 0 && bt.count[c] > max_leaf; };
+    auto area_of = [&](int32_t c) {  // of an internal child: the only kind that is opened
+        if (c < 0) return -1.0f;
+        float bx[6];
+        load_box(bt, c, bx);
+        return box_area(bx);
+    };
+    float area[W];
+    bool large[W];
+    for (int k = 0; k < 2; ++k) {
+        area[k] = area_of(kid[k]);
+        large[k] = opens(kid[k]);
+    }
     bool fill = false;  // every child fits a leaf: open leaf-sized internal children into the free slots
     while (m < W) {
         int best = -1;
         float best_area = -1.0f;
         for (int k = 0; k < m; ++k) {
-            if (!(fill ? kid[k] >= 0 : opens(kid[k]))) continue;
-            float bx[6];
-            load_box(bt, kid[k], bx);
-            const float ar = box_area(bx);
-            if (ar > best_area) {
-                best_area = ar;
+            if (!(fill ? kid[k] >= 0 : large[k])) continue;
+            if (area[k] > best_area) {
+                best_area = area[k];
                 best = k;
             }
         }
@@ -203,16 +240,21 @@ __global__ void k_collapse(int nq, const int4* __restrict__ q_in, int4* __restri
         kid[best] = bt.left[c];
         kid[m] = bt.right[c];
         start[m] = s + ref_count(bt, kid[best]);
+        for (const int k : {best, m}) {
+            area[k] = area_of(kid[k]);
+            large[k] = opens(kid[k]);
+        }
         ++m;
     }
     int inner = 0;
-    for (int k = 0; k < m; ++k) inner += opens(kid[k]) ? 1 : 0;
+    for (int k = 0; k < m; ++k) inner += large[k] ? 1 : 0;
     const int base = inner ? atomicAdd(&cs->nodes, inner) : 0;
+    int leaf_at = inner < m ? atomicAdd(&cs->leaves, m - inner) : 0;
     constexpr int Q = W / 4;
     constexpr int F4 = W == 8 ? NodeShape<8>::kF4 : NodeShape<4>::kF4;
     float* node = reinterpret_cast<float*>(nodes + int64_t(item.y) * F4);
     int32_t* ch = reinterpret_cast<int32_t*>(node + 6 * Q * 4);
-    int k_in = 0, n_leaf = 0;
+    int k_in = 0;
     for (int j = 0; j < W; ++j) {
         if (j >= m) {
             for (int a = 0; a < 3; ++a) {
@@ -229,25 +271,19 @@ __global__ void k_collapse(int nq, const int4* __restrict__ q_in, int4* __restri
             node[(2 * a) * Q * 4 + j] = bx[a];
             node[(2 * a + 1) * Q * 4 + j] = bx[3 + a];
         }
-        if (opens(c)) {
+        if (large[j]) {
             const int w = base + k_in++;
             ch[j] = w;
             q_out[w - next_base] = make_int4(c, w, start[j], 0);
         } else {
-            const int32_t s = start[j], k = ref_count(bt, c);
-            ch[j] = int32_t(uint32_t(s) | 0x80000000u);
-            leaf_slots(bt, c, s, k, perm);
-            last[s + k - 1] = 1;
-            ++n_leaf;
+            ch[j] = int32_t(uint32_t(start[j]) | 0x80000000u);
+            leaves[leaf_at++] = make_int2(c, start[j]);
         }
     }
     if (W == 4) {  // the layout's padding
         for (int k = 28; k < 32; ++k) node[k] = 0.0f;
     }
-    if (n_leaf) {
-        atomicAdd(&cs->leaves, n_leaf);
-        atomicMax(&cs->depth, level + 2);
-    }
+    if (inner < m) atomicMax(&cs->depth, level + 2);
 }
 
 // Device buffers of the Morton stage. Declare after the build's ScratchScope.
@@ -323,7 +359,7 @@ inline void morton_prims(MortonPrims& m, const float* tri, int64_t n, cudaStream
 
 // Collapses the binary tree rooted at internal node `root` (n > max_leaf) into
 // t's W-wide device nodes; fills perm (leaf slot -> primitive) and last.
-// Returns the number of levels (one launch each).
+// Returns the number of levels (one launch each, and one to fill the leaves).
 inline int collapse_wide(BuiltTree& t, const BinaryTree& bt, int32_t root, int W, int max_leaf, int32_t* perm,
                          uint8_t* last, cudaStream_t st) {
     const int F4 = W == 8 ? NodeShape<8>::kF4 : NodeShape<4>::kF4;
@@ -332,6 +368,8 @@ inline int collapse_wide(BuiltTree& t, const BinaryTree& bt, int32_t root, int W
     *h_cs.p = CollapseState{1, 1, 0, 0};
     DevBuf<CollapseState> d_cs;
     DevBuf<int4> d_qa, d_qb;
+    DevBuf<int2> d_leaves;
+    d_leaves.alloc(size_t(bt.n));  // a leaf holds at least one primitive
     DevBuf<float4> d_wide;
     d_cs.alloc(1);
     check(cudaMemcpyAsync(d_cs.p, h_cs.p, sizeof(CollapseState), cudaMemcpyHostToDevice, st), "collapse state");
@@ -358,11 +396,11 @@ inline int collapse_wide(BuiltTree& t, const BinaryTree& bt, int32_t root, int W
         d_qb.alloc(size_t(nq) * W);
         const int next_base = allocated;
         if (W == 8)
-            k_collapse<8><<<grid(nq, 128), 128, 0, st>>>(nq, d_qa.p, d_qb.p, next_base, levels, max_leaf, bt, last,
-                                                        perm, d_cs.p, d_wide.p);
+            k_collapse<8><<<grid(nq, 128), 128, 0, st>>>(nq, d_qa.p, d_qb.p, next_base, levels, max_leaf, bt,
+                                                        d_leaves.p, d_cs.p, d_wide.p);
         else
-            k_collapse<4><<<grid(nq, 128), 128, 0, st>>>(nq, d_qa.p, d_qb.p, next_base, levels, max_leaf, bt, last,
-                                                        perm, d_cs.p, d_wide.p);
+            k_collapse<4><<<grid(nq, 128), 128, 0, st>>>(nq, d_qa.p, d_qb.p, next_base, levels, max_leaf, bt,
+                                                        d_leaves.p, d_cs.p, d_wide.p);
         check(cudaGetLastError(), "collapse");
         check(cudaMemcpyAsync(h_cs.p, d_cs.p, sizeof(CollapseState), cudaMemcpyDeviceToHost, st), "level");
         check(cudaStreamSynchronize(st), "level");
@@ -371,6 +409,8 @@ inline int collapse_wide(BuiltTree& t, const BinaryTree& bt, int32_t root, int W
         allocated = h_cs.p->nodes;
         swap_bufs(d_qa, d_qb);
     }
+    k_fill_leaves<<<grid(h_cs.p->leaves), 256, 0, st>>>(h_cs.p->leaves, d_leaves.p, bt, last, perm);
+    check(cudaGetLastError(), "leaf slots");
     t.root = 0;
     t.depth = h_cs.p->depth;
     t.leaves = h_cs.p->leaves;
