@@ -1181,8 +1181,8 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
     DevBuf<DShape> d_shapes;
     DevBuf<int> d_cnt_next, d_off_next, d_cnt_shape, d_off_shape;
     DevBuf<BuildState> d_state;
-    PinnedBuf<int> h_scene;
-    PinnedBuf<BuildState> h_state;
+    int h_scene[6];
+    BuildState h_state;
     const int64_t nn = std::max<int64_t>(n, 1);
     d_tri.alloc(size_t(std::max<int64_t>(nt, 1)) * 9);
     DevBuf<float> d_extra;
@@ -1199,13 +1199,11 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
     d_pr.alloc(size_t(nn));
     d_scene.alloc(6);
     d_state.alloc(1);
-    h_scene.alloc(6);
-    h_state.alloc(1);
 
     // Scene box (core/scene.cpp:146-154): union of the primitive boxes, enlarged by 0.1%.
     Box scene;
     {
-        empty_box(h_scene.p);
+        empty_box(h_scene);
         if (n > 0) {
             if (nt > 0) {
                 check(upload_host(d_tri.p, tri, size_t(nt) * 9 * sizeof(float), st), "upload");
@@ -1219,13 +1217,13 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
                 k_box_setup<<<grid(p.nextra), 256, 0, st>>>(d_extra.p, nt, p.nextra, n, d_cx.p, d_cy.p, d_cz.p,
                                                             d_idx.p, d_pb.p);
             }
-            check(cudaMemcpyAsync(d_scene.p, h_scene.p, 6 * sizeof(int), cudaMemcpyHostToDevice, st), "scene box");
+            check(cudaMemcpyAsync(d_scene.p, h_scene, 6 * sizeof(int), cudaMemcpyHostToDevice, st), "scene box");
             k_scene_box<<<std::min<unsigned>(grid(n), 148 * 8), 256, 0, st>>>(n, d_pb.p, d_scene.p);
             check(cudaGetLastError(), "primitive setup");
-            check(cudaMemcpyAsync(h_scene.p, d_scene.p, 6 * sizeof(int), cudaMemcpyDeviceToHost, st), "scene box");
+            check(cudaMemcpyAsync(h_scene, d_scene.p, 6 * sizeof(int), cudaMemcpyDeviceToHost, st), "scene box");
             check(cudaStreamSynchronize(st), "primitive setup");
         }
-        scene = box_from_images(h_scene.p);
+        scene = box_from_images(h_scene);
         const float threshold = 0.001f;
         float delta[3];
         for (int k = 0; k < 3; ++k) delta[k] = (scene.mx[k] - scene.mn[k]) * threshold;
@@ -1264,8 +1262,8 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
     }
     const bool root_node = n > p.max_leaf && p.max_depth != 1;
     const bool large_root = root_node && n > kSmall, small_root = root_node && !large_root;
-    *h_state.p = BuildState{large_root ? 1 : 0, 1, root_node ? 0 : 1, 0, 0, 0, {small_root ? 1 : 0, 0}};
-    check(cudaMemcpyAsync(d_state.p, h_state.p, sizeof(BuildState), cudaMemcpyHostToDevice, st), "state");
+    h_state = BuildState{large_root ? 1 : 0, 1, root_node ? 0 : 1, 0, 0, 0, {small_root ? 1 : 0, 0}};
+    check(cudaMemcpyAsync(d_state.p, &h_state, sizeof(BuildState), cudaMemcpyHostToDevice, st), "state");
     DNode root{};
     SmallNode root_small{};
     if (root_node) {
@@ -1317,9 +1315,9 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
             swap_bufs(d_cur, d_next);
         }
         queued += kGroup;
-        check(cudaMemcpyAsync(h_state.p, d_state.p, sizeof(BuildState), cudaMemcpyDeviceToHost, st), "state");
+        check(cudaMemcpyAsync(&h_state, d_state.p, sizeof(BuildState), cudaMemcpyDeviceToHost, st), "state");
         check(cudaStreamSynchronize(st), "split rounds");
-        if (h_state.p->na == 0) break;
+        if (h_state.na == 0) break;
         if (queued > max_rounds) throw std::runtime_error("GPU build: the split rounds did not finish");
     }
     // The small nodes, one pass per level of the tree (a node's children are one
@@ -1328,7 +1326,7 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
     if (root_node) {
         int in = 0;
         for (;;) {
-            const int count = h_state.p->small[in];
+            const int count = h_state.small[in];
             if (count == 0) break;
             if (++passes > p.max_depth) throw std::runtime_error("GPU build: the small splits did not finish");
             k_split_small<<<std::min<unsigned>(grid(count, kSmallWarps), 148 * 16), 32 * kSmallWarps, 0, st>>>(
@@ -1338,11 +1336,11 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
             check(cudaGetLastError(), "small splits");
             swap_bufs(d_small, d_small_next);
             in ^= 1;
-            check(cudaMemcpyAsync(h_state.p, d_state.p, sizeof(BuildState), cudaMemcpyDeviceToHost, st), "state");
+            check(cudaMemcpyAsync(&h_state, d_state.p, sizeof(BuildState), cudaMemcpyDeviceToHost, st), "state");
             check(cudaStreamSynchronize(st), "small splits");
         }
     }
-    const BuildState fin = *h_state.p;
+    const BuildState fin = h_state;
     const int shape_count = fin.shapes;
     t.depth = fin.depth_max;
 

@@ -194,7 +194,7 @@ BuiltTree build_tree_ploc(const float* tri, int64_t ntri, const BuildParams& p, 
     DevBuf<int4> d_rec[2];
     DevBuf<uint32_t> d_keep, d_pos, d_scan;
     DevBuf<int> d_ctr;
-    PinnedBuf<int> h_ctr;
+    int h_ctr[2];
     const int32_t* perm = m.sorted.p;  // one leaf: Morton order
     if (n <= p.max_leaf) {
         single_leaf(t, n, d_last.p, st);
@@ -211,7 +211,6 @@ BuiltTree build_tree_ploc(const float* tri, int64_t ntri, const BuildParams& p, 
         d_pos.alloc(size_t(n));
         d_scan.alloc(std::max<size_t>(psort::scan_scratch_words(size_t(n)), 8));  // covers every smaller count too
         d_ctr.alloc(2);  // [0] internal nodes made, [1] clusters left
-        h_ctr.alloc(4);
         d_perm.alloc(size_t(n));
         check(cudaMemsetAsync(d_ctr.p, 0, 2 * sizeof(int), st), "counters");
         k_ploc_init<<<grid(n), 256, 0, st>>>(n, m.sorted.p, m.pb.p, d_rec[0].p);
@@ -227,16 +226,16 @@ BuiltTree build_tree_ploc(const float* tri, int64_t ntri, const BuildParams& p, 
             k_ploc_compact<<<grid(nc), 256, 0, st>>>(nc, d_rec[cur].p, d_keep.p, d_pos.p, d_rec[1 - cur].p,
                                                      d_ctr.p + 1);
             check(cudaGetLastError(), "cluster compaction");
-            check(cudaMemcpyAsync(h_ctr.p, d_ctr.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st), "cluster count");
+            check(cudaMemcpyAsync(h_ctr, d_ctr.p, 2 * sizeof(int), cudaMemcpyDeviceToHost, st), "cluster count");
             check(cudaStreamSynchronize(st), "cluster count");
             launches += 4 + (nc > psort::kScanTile ? 3 : 1);  // search, merge, scan, compaction
             ++iterations;
-            if (h_ctr.p[1] >= nc || h_ctr.p[1] < 1)
+            if (h_ctr[1] >= nc || h_ctr[1] < 1)
                 throw std::runtime_error("PLOC iteration merged no clusters");
-            nc = h_ctr.p[1];
+            nc = h_ctr[1];
             cur = 1 - cur;
         }
-        if (h_ctr.p[0] != ni) throw std::runtime_error("PLOC made a wrong number of internal nodes");
+        if (h_ctr[0] != ni) throw std::runtime_error("PLOC made a wrong number of internal nodes");
         int4 root_rec;
         check(cudaMemcpyAsync(&root_rec, d_rec[cur].p, sizeof(int4), cudaMemcpyDeviceToHost, st), "root");
         check(cudaStreamSynchronize(st), "root");

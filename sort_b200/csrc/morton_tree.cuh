@@ -293,7 +293,7 @@ struct MortonPrims {
     DevBuf<uint64_t> keys, keys_sorted;
     DevBuf<int> box;
     DevBuf<unsigned char> temp;
-    PinnedBuf<int> h_box;
+    int h_box[12];
     Box scene{};
     int launches = 0;
 };
@@ -310,21 +310,20 @@ inline void morton_prims(MortonPrims& m, const float* tri, int64_t n, cudaStream
     m.pb.alloc(size_t(nn) * 6);
     m.idx.alloc(size_t(nn));
     m.box.alloc(12);
-    m.h_box.alloc(12);
-    empty_box(m.h_box.p);
-    empty_box(m.h_box.p + 6);
+    empty_box(m.h_box);
+    empty_box(m.h_box + 6);
     if (n > 0) {
         check(upload_host(m.tri.p, tri, size_t(n) * 9 * sizeof(float), st), "upload");
         k_prim_setup<<<grid(n), 256, 0, st>>>(m.tri.p, n, n, m.cx.p, m.cy.p, m.cz.p, m.idx.p, m.pb.p);
-        check(cudaMemcpyAsync(m.box.p, m.h_box.p, 12 * sizeof(int), cudaMemcpyHostToDevice, st), "boxes");
+        check(cudaMemcpyAsync(m.box.p, m.h_box, 12 * sizeof(int), cudaMemcpyHostToDevice, st), "boxes");
         const unsigned gb = std::min<unsigned>(grid(n), 148 * 8);
         k_scene_box<<<gb, 256, 0, st>>>(n, m.pb.p, m.box.p);
         k_centroid_box<<<gb, 256, 0, st>>>(n, m.cx.p, m.cy.p, m.cz.p, m.box.p + 6);
         check(cudaGetLastError(), "primitive setup");
-        check(cudaMemcpyAsync(m.h_box.p, m.box.p, 12 * sizeof(int), cudaMemcpyDeviceToHost, st), "boxes");
+        check(cudaMemcpyAsync(m.h_box, m.box.p, 12 * sizeof(int), cudaMemcpyDeviceToHost, st), "boxes");
         check(cudaStreamSynchronize(st), "primitive setup");
     }
-    Box scene = box_from_images(m.h_box.p);
+    Box scene = box_from_images(m.h_box);
     const float threshold = 0.001f;
     float delta[3];
     for (int k = 0; k < 3; ++k) delta[k] = (scene.mx[k] - scene.mn[k]) * threshold;
@@ -363,16 +362,14 @@ inline void morton_prims(MortonPrims& m, const float* tri, int64_t n, cudaStream
 inline int collapse_wide(BuiltTree& t, const BinaryTree& bt, int32_t root, int W, int max_leaf, int32_t* perm,
                          uint8_t* last, cudaStream_t st) {
     const int F4 = W == 8 ? NodeShape<8>::kF4 : NodeShape<4>::kF4;
-    PinnedBuf<CollapseState> h_cs;
-    h_cs.alloc(1);
-    *h_cs.p = CollapseState{1, 1, 0, 0};
+    CollapseState h_cs{1, 1, 0, 0};
     DevBuf<CollapseState> d_cs;
     DevBuf<int4> d_qa, d_qb;
     DevBuf<int2> d_leaves;
     d_leaves.alloc(size_t(bt.n));  // a leaf holds at least one primitive
     DevBuf<float4> d_wide;
     d_cs.alloc(1);
-    check(cudaMemcpyAsync(d_cs.p, h_cs.p, sizeof(CollapseState), cudaMemcpyHostToDevice, st), "collapse state");
+    check(cudaMemcpyAsync(d_cs.p, &h_cs, sizeof(CollapseState), cudaMemcpyHostToDevice, st), "collapse state");
     size_t wide_cap = size_t(std::max<int64_t>(64, bt.n / 16));
     d_wide.alloc(wide_cap * F4);
     d_qa.alloc(64);
@@ -402,18 +399,18 @@ inline int collapse_wide(BuiltTree& t, const BinaryTree& bt, int32_t root, int W
             k_collapse<4><<<grid(nq, 128), 128, 0, st>>>(nq, d_qa.p, d_qb.p, next_base, levels, max_leaf, bt,
                                                         d_leaves.p, d_cs.p, d_wide.p);
         check(cudaGetLastError(), "collapse");
-        check(cudaMemcpyAsync(h_cs.p, d_cs.p, sizeof(CollapseState), cudaMemcpyDeviceToHost, st), "level");
+        check(cudaMemcpyAsync(&h_cs, d_cs.p, sizeof(CollapseState), cudaMemcpyDeviceToHost, st), "level");
         check(cudaStreamSynchronize(st), "level");
         ++levels;
-        nq = h_cs.p->nodes - next_base;
-        allocated = h_cs.p->nodes;
+        nq = h_cs.nodes - next_base;
+        allocated = h_cs.nodes;
         swap_bufs(d_qa, d_qb);
     }
-    k_fill_leaves<<<grid(h_cs.p->leaves), 256, 0, st>>>(h_cs.p->leaves, d_leaves.p, bt, last, perm);
+    k_fill_leaves<<<grid(h_cs.leaves), 256, 0, st>>>(h_cs.leaves, d_leaves.p, bt, last, perm);
     check(cudaGetLastError(), "leaf slots");
     t.root = 0;
-    t.depth = h_cs.p->depth;
-    t.leaves = h_cs.p->leaves;
+    t.depth = h_cs.depth;
+    t.leaves = h_cs.leaves;
     t.n_interior = allocated;
     // The scene owns its nodes: an exact-size copy outside the scratch pool.
     float4* nodes = nullptr;
