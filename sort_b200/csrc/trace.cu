@@ -222,18 +222,24 @@ static cudaError_t launch_walk(const TraceLaunch& L, const DevTree& tr, const De
     const int refill = L.tuning.schedule == kSchedulePersistent ? L.tuning.refill_threshold : Shape::kRefill;
     // A large launch takes its rays from a counter: the caller's, or one from the
     // scratch pool (not while the stream is captured: a graph may be replayed
-    // beside itself, and callers that asked for no scratch get none).
+    // beside itself, and callers that asked for no scratch get none). Without the
+    // memory for one the launch goes by spans, as those do: 2.68 against 2.15 ms
+    // on 4M diffuse rays.
     char* scratch = nullptr;
-    cudaMemPool_t pool = nullptr;
     if (!counter && L.scratch && !L.n_dev && n > (int64_t)slots * 32) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
             (void)cudaGetLastError();
             cap = cudaStreamCaptureStatusActive;
         }
-        if (cap == cudaStreamCaptureStatusNone && (pool = trace_scratch_pool(dev)) != nullptr) {
-            if ((e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), 256, pool, s)) != cudaSuccess) return e;
-            counter = reinterpret_cast<unsigned*>(scratch);
+        if (cap == cudaStreamCaptureStatusNone) {
+            cudaMemPool_t pool = trace_scratch_pool(dev);
+            if (pool && cudaMallocFromPoolAsync(reinterpret_cast<void**>(&scratch), 256, pool, s) == cudaSuccess) {
+                counter = reinterpret_cast<unsigned*>(scratch);
+            } else {
+                (void)cudaGetLastError();
+                scratch = nullptr;
+            }
         }
     }
     for (int64_t a = 0; a < n && e == cudaSuccess; a += kMaxWalkRays) {
