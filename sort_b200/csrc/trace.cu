@@ -27,6 +27,7 @@
 #include <mutex>
 #include <vector>
 
+#include "group_walk.cuh"
 #include "prefix_sort.cuh"
 #include "trace_kernels.h"
 #include "traversal.cuh"
@@ -87,6 +88,14 @@ struct WalkShape {
     static constexpr int kBlocks = W == 8 && !Q8 ? 7 : 8;
     static constexpr int kRefill = Q8 ? 12 : 24;
 };
+
+// Launch shape of k_trace_groups: blocks of 128 per SM (56 registers). A launch of at
+// most a ray per group (18,944 rays on 148 SMs) over a width-8 tree takes it.
+// k_trace_walk against it, us: diffuse rays, 5.2M triangles, 84.6 / 77.7 at 18,944
+// rays, 94.6 / 92.0 at 26,000, 110 / 172 at 65,536; shadow 67.0 / 51.3, 91.4 / 66.4,
+// 95.8 / 129; camera, 82k triangles, 32.9 / 30.8 at 18,944. A larger launch is bound
+// by issue slots, of which this form takes more.
+constexpr int kGroupBlocks = 8;
 
 // Rays of a launch as its warps take them: one span of `span` rays per warp, or,
 // with a counter, as many as the warp has idle lanes from the launch's counter,
@@ -186,6 +195,60 @@ __global__ void __launch_bounds__(kWalkThreads, WalkShape<W, Q8>::kBlocks)
     walk_rays<W, ANY, STACK, Q8, false>(job, shared + (threadIdx.x >> 5), lane, refill, err);
 }
 
+// Traces min(n, *n_dev) rays (n_dev may be null) with eight lanes per ray; up to a ray
+// per warp each warp has one.
+template <bool ANY, int STACK, bool Q8>
+__global__ void __launch_bounds__(kWalkThreads, kGroupBlocks)
+    k_trace_groups(const __grid_constant__ DevTree tr, const __grid_constant__ DevRays rays, int n,
+                   int32_t* __restrict__ prim_out, float* __restrict__ t_out, float* __restrict__ u_out,
+                   float* __restrict__ v_out, uint8_t* __restrict__ occ_out, int* __restrict__ err,
+                   const int* __restrict__ n_dev) {
+    __shared__ GroupStack<ANY, STACK> stacks[kBlockGroups];
+    const int lane = threadIdx.x & 31, warp = (int)blockIdx.x * kWalkWarps + (threadIdx.x >> 5);
+    const int ord = lane & (kGroupLanes - 1), g = lane / kGroupLanes;
+    if (n_dev) n = min(n, *n_dev);
+    const int warps = (int)gridDim.x * kWalkWarps;
+    const int share = min(kWarpGroups, (n + warps - 1) / warps);  // groups of a warp that take rays
+    int i = -1, next = g < share ? warp * share + g : n;
+    GroupWalk<ANY, STACK, Q8> w;
+    w.cur = kEmpty;
+    for (;;) {
+        const bool idle = w.cur == kEmpty && (i >= 0 || next < n);
+        if (__any_sync(kFullWarp, idle)) {
+            if (idle) {
+                if (i >= 0) {
+                    if constexpr (ANY) {
+                        if (ord == 0) occ_out[i] = w.prim >= 0 ? 1 : 0;
+                    } else {
+                        if (ord == 0) prim_out[i] = w.prim;
+                        if (ord == 1) t_out[i] = w.t;
+                        if (ord == 2 && u_out) u_out[i] = w.u;
+                        if (ord == 3 && v_out) v_out[i] = w.v;
+                    }
+                    i = -1;
+                }
+                if (next < n) {
+                    i = next;
+                    next += warps * share;
+                    RayState r;
+                    r.o[0] = rays.ox[i];
+                    r.o[1] = rays.oy[i];
+                    r.o[2] = rays.oz[i];
+                    r.d[0] = rays.dx[i];
+                    r.d[1] = rays.dy[i];
+                    r.d[2] = rays.dz[i];
+                    r.tmin = rays.tmin[i];
+                    r.tmax = rays.tmax[i];
+                    w.begin(tr, r);
+                }
+            }
+        } else if (__all_sync(kFullWarp, w.cur == kEmpty)) {
+            break;
+        }
+        w.step(tr.nodes, tr.tris, &stacks[(threadIdx.x >> 5) * kWarpGroups + g], lane, err);
+    }
+}
+
 // Stream-ordered scratch of a launch (the sorted schedule's keys and order, the
 // ray counter): one pool per device that keeps up to 1 GiB mapped between
 // launches (NULL if it cannot be made).
@@ -209,7 +272,8 @@ static cudaMemPool_t trace_scratch_pool(int device) {
     return pools[size_t(device)];
 }
 
-// Launches k_trace_walk over n rays, with the launch's counter or without one.
+// Launches k_trace_walk over n rays, with the launch's counter or without one, or
+// k_trace_groups where there are few.
 template <int W, bool ANY, int STACK, bool Q8>
 static cudaError_t launch_walk(const TraceLaunch& L, const DevTree& tr, const DevRays& rays, int64_t n,
                                const int32_t* order, unsigned* counter, cudaStream_t s) {
@@ -219,6 +283,15 @@ static cudaError_t launch_walk(const TraceLaunch& L, const DevTree& tr, const De
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     const int slots = (sms < 1 ? 1 : sms) * Shape::kBlocks * kWalkWarps;
+    if constexpr (W == 8) {
+        const int group_warps = (sms < 1 ? 1 : sms) * kGroupBlocks * kWalkWarps;
+        if (!order && n <= (int64_t)group_warps * kWarpGroups) {
+            const int warps = n < group_warps ? (int)n : group_warps;
+            k_trace_groups<ANY, STACK, Q8><<<(unsigned)((warps + kWalkWarps - 1) / kWalkWarps), kWalkThreads, 0, s>>>(
+                tr, rays, (int)n, L.prim, L.t, L.u, L.v, L.occ, L.err, L.n_dev);
+            return cudaGetLastError();
+        }
+    }
     const int refill = L.tuning.schedule == kSchedulePersistent ? L.tuning.refill_threshold : Shape::kRefill;
     // A large launch takes its rays from a counter: the caller's, or one from the
     // scratch pool (not while the stream is captured: a graph may be replayed
