@@ -459,20 +459,31 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
     // one shadow queue of 2 entries per path (rays + contributions), occlusion
     // flags, throughput and radiance, shadow entries, counts; then the shared ray
     // totals.
-    const int per_wave = sg::wave_samples(P, sg::kWavePaths, spp), waves = (spp + per_wave - 1) / per_wave;
-    const int in_flight = waves < sg::kInFlight ? waves : sg::kInFlight;
-    const size_t cap = (size_t)P * per_wave, scap = 2 * cap;
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    const size_t qbytes = align(cap * 8 * 4) + align(cap * 4);
-    const size_t set = 2 * qbytes + align(cap * 4) * 2 + align(scap * 8 * 4) + align(scap * 3 * 4) + align(scap) +
-                       align(cap * 6 * 4) + align(cap * 2 * 4) + align(sg::kWaveCounts * sizeof(sg::WaveCount));
-    const size_t need = in_flight * set + align(16);
-    if (ps->buf_bytes < need) {
+    int per_wave = sg::wave_samples(P, sg::kWavePaths, spp), waves, in_flight;
+    size_t cap, scap, need;
+    for (;;) {
+        waves = (spp + per_wave - 1) / per_wave;
+        in_flight = waves < sg::kInFlight ? waves : sg::kInFlight;
+        cap = (size_t)P * per_wave;
+        scap = 2 * cap;
+        const size_t qbytes = align(cap * 8 * 4) + align(cap * 4);
+        const size_t set = 2 * qbytes + align(cap * 4) * 2 + align(scap * 8 * 4) + align(scap * 3 * 4) + align(scap) +
+                           align(cap * 6 * 4) + align(cap * 2 * 4) + align(sg::kWaveCounts * sizeof(sg::WaveCount));
+        need = in_flight * set + align(16);
+        if (ps->buf_bytes >= need) break;
         if (ps->d_buf) cudaFree(ps->d_buf);
         ps->d_buf = nullptr;
+        ps->d_totals = nullptr;
         ps->buf_bytes = 0;
-        if ((e = cudaMalloc(&ps->d_buf, need)) != cudaSuccess) return pt_fail(e);
-        ps->buf_bytes = need;
+        e = cudaMalloc(&ps->d_buf, need);
+        if (e == cudaSuccess) {
+            ps->buf_bytes = need;
+            break;
+        }
+        if (e != cudaErrorMemoryAllocation || per_wave == 1) return pt_fail(e);
+        (void)cudaGetLastError();  // fewer samples share a wave: less memory, the same image
+        per_wave = (per_wave + 1) / 2;
     }
     char* b = (char*)ps->d_buf;
     auto take = [&](size_t bytes) {
