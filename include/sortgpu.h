@@ -400,7 +400,7 @@ sg_status sg_trace_any_host(const sg_scene* scene, const float* rays8, int64_t n
  * take the allocator's locks or wait on an implicit synchronisation). Rays and hits are staged in a 24 MiB array compiled into
  * the library, held on every GPU that loads it until exit; at most 524,288 rays
  * per call (SG_ERR_LIMIT beyond). All calls share that array, so calls whose
- * work overlaps on the GPU race. Every batch runs one ray per thread, whatever
+ * work overlaps on the GPU race. Every batch runs in batch order, whatever
  * schedule sg_scene_set_tuning chose (the sorted schedule would take scratch
  * from a pool); results are the same under every schedule. Scenes with hair
  * lines are rejected (SG_ERR_UNSUPPORTED). The first call on a device looks up

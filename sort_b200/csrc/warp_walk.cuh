@@ -20,14 +20,14 @@
 //    idle, so the node visits run with 25 lanes;
 //  * a node's children go through packed FP32 pairs, one 32-byte load per plane,
 //    and the two nearest hits stay in registers (a push is a predicated store).
-// That issues 11.4k instructions per 32 rays at 24.9 lanes. The L1 data pipe is
-// the next limit (77% of its peak on diffuse rays, 87% on shadow rays: a
-// divergent 32-byte load per plane and lane, 48 bytes per triangle), beside 5.6
-// warps waiting on loads per issue; DRAM is at 10%.
-// Measured on one box, start to now: 4,194,304 diffuse rays, 21M triangles, sort
-// included 3.93 -> 2.50 ms; as many shadow rays 3.61 -> 2.09 ms; 1,048,576 camera
-// rays, 82k triangles, width 4, 0.255 -> 0.182 ms; 700,001 diffuse rays, 1.3M
-// triangles, 8-bit nodes 0.744 -> 0.323 ms; 4,099 camera rays 68 -> 29 us.
+// That issues 11.5k instructions per 32 rays at 24.6 lanes (shadow rays 10.2k at
+// 25.9). Issue slots are then 60% busy and the L1 data pipe is at 73% of its peak
+// (shadow 83%: a divergent 32-byte load per plane and lane, 48 bytes per
+// triangle), with 4.7 warps waiting on loads per issue (5.8); DRAM is at 2%.
+// Before and now, one box: 4,194,304 diffuse rays, 21M triangles, 3.93 ms in sorted
+// order, now 2.15 in batch order; as many shadow rays 3.61 -> 2.05; 1,048,576 camera
+// rays, 82k triangles, width 4, 0.255 -> 0.176; 700,001 diffuse rays, 1.3M
+// triangles, 8-bit nodes 0.744 -> 0.323.
 // Slower forms: a second round's triangles fetched ahead (52 bytes spilled,
 // 2.99 ms on the diffuse rays against 2.66), every hit but the nearest pushed and
 // sorted on the stack (2.98), the 1/d and -o/d pairs kept doubled in registers
