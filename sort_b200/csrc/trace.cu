@@ -35,31 +35,8 @@
 
 namespace sg {
 
-// One ray per thread for the whole launch. With n_dev set, the batch size is
-// min(n, *n_dev), read on the device (queues whose length only the GPU knows).
-// Q8 reads 8-bit nodes.
-// With `order` set, thread k traces ray order[k] (the sorted schedule).
-template <int W, bool ANY, int STACK, bool STATS, bool Q8>
-__device__ __forceinline__ void trace_one_ray(const DevTree& tr, const DevRays& rays, int64_t n,
-                                              int32_t* __restrict__ prim_out, float* __restrict__ t_out,
-                                              float* __restrict__ u_out, float* __restrict__ v_out,
-                                              uint8_t* __restrict__ occ_out, int* __restrict__ err,
-                                              unsigned long long* __restrict__ stats, const int* __restrict__ n_dev,
-                                              const int32_t* __restrict__ order) {
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n_dev && k >= (int64_t)*n_dev) return;
-    if (k >= n) return;
-    const int64_t i = order ? (int64_t)__ldg(order + k) : k;
-    Traversal<W, ANY, STACK, STATS, Q8, true> tv;
-    uint2 stk_mem[STACK];
-    tv.stk = stk_mem;
-    if (tv.start(tr, rays, i))
-        while (!tv.step(tr, err)) {
-        }
-    tv.finish(i, prim_out, t_out, u_out, v_out, occ_out, stats);
-}
-
-// The counting launches' kernel.
+// The counting launches' kernel: one ray per thread (`Traversal`). With n_dev set, the
+// batch size is min(n, *n_dev), read on the device. Q8 reads 8-bit nodes.
 template <int W, bool ANY, int STACK, bool Q8>
 __global__ void __launch_bounds__(128, 9) k_trace_stats(DevTree tr, DevRays rays, int64_t n,
                                                         int32_t* __restrict__ prim_out, float* __restrict__ t_out,
@@ -67,8 +44,15 @@ __global__ void __launch_bounds__(128, 9) k_trace_stats(DevTree tr, DevRays rays
                                                         uint8_t* __restrict__ occ_out, int* __restrict__ err,
                                                         unsigned long long* __restrict__ stats,
                                                         const int* __restrict__ n_dev) {
-    trace_one_ray<W, ANY, STACK, true, Q8>(tr, rays, n, prim_out, t_out, u_out, v_out, occ_out, err, stats, n_dev,
-                                           nullptr);
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if ((n_dev && i >= (int64_t)*n_dev) || i >= n) return;
+    Traversal<W, ANY, STACK, true, Q8, true> tv;
+    uint2 stk_mem[STACK];
+    tv.stk = stk_mem;
+    if (tv.start(tr, rays, i))
+        while (!tv.step(tr, err)) {
+        }
+    tv.finish(i, prim_out, t_out, u_out, v_out, occ_out, stats);
 }
 
 // Launch shape of k_trace_walk per tree form: blocks of 128 per SM (registers:
