@@ -353,8 +353,8 @@ cudaError_t pt_scale(float* image, int64_t n, float s, cudaStream_t st) {
 cudaError_t pt_wave(const PtDev& dev, const TraceLaunch& base_in, const DevTree& tree, const Cam& cam, int width,
                     int height, int p0, int n, uint2 key, int sample, int samples, int max_depth, const PtWave& w,
                     float* image, cudaStream_t s) {
+    if (n <= 0 || samples <= 0 || (int64_t)n * samples > w.cap || w.cap > kMaxWavePaths) return cudaErrorInvalidValue;
     const int cap = w.cap, scap = 2 * w.cap;
-    if (n <= 0 || samples <= 0 || (int64_t)n * samples > cap) return cudaErrorInvalidValue;
     const int paths = n * samples;
     TraceLaunch base = base_in;
     base.tuning.schedule = kScheduleThreadPerRay;  // queue lengths live on the device
@@ -460,12 +460,15 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
     // flags, throughput and radiance, shadow entries, counts; then the shared ray
     // totals.
     auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    int per_wave = sg::wave_samples(P, sg::kWavePaths, spp), waves, in_flight;
+    // A frame too large for one wave goes in parts of `part` pixels.
+    const int part = (int)std::min<int64_t>(P, sg::kMaxWavePaths), parts = (P + part - 1) / part;
+    int per_wave = sg::wave_samples(P, sg::kWavePaths, spp), in_flight;
+    int64_t waves;
     size_t cap, scap, need;
     for (;;) {
-        waves = (spp + per_wave - 1) / per_wave;
-        in_flight = waves < sg::kInFlight ? waves : sg::kInFlight;
-        cap = (size_t)P * per_wave;
+        waves = (int64_t)((spp + per_wave - 1) / per_wave) * parts;
+        in_flight = waves < sg::kInFlight ? (int)waves : sg::kInFlight;
+        cap = (size_t)part * per_wave;
         scap = 2 * cap;
         const size_t qbytes = align(cap * 8 * 4) + align(cap * 4);
         const size_t set = 2 * qbytes + align(cap * 4) * 2 + align(scap * 8 * 4) + align(scap * 3 * 4) + align(scap) +
@@ -537,13 +540,14 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
     if ((e = cudaEventRecord(ps->begun, s)) != cudaSuccess) return pt_fail(e);
     for (int k = 1; k < sg::kInFlight; ++k)
         if ((e = cudaStreamWaitEvent(ps->extra[k], ps->begun, 0)) != cudaSuccess) return pt_fail(e);
-    for (int k = 0; k < waves; ++k) {
-        const int set = k % sg::kInFlight, first = k * per_wave;
+    for (int64_t k = 0; k < waves; ++k) {
+        const int set = int(k % sg::kInFlight), first = int(k / parts) * per_wave, from = int(k % parts) * part;
         sg::PtWave& ws = w[set];
         ws.flush_after = k > 0 ? ps->flushed[(k - 1) % sg::kInFlight] : nullptr;  // image sums in order
         const cudaStream_t on = set ? ps->extra[set] : s;
-        if ((e = sg::pt_wave(dev, base, tree, cam, width, height, p0, P, key, first, std::min(per_wave, spp - first),
-                             max_depth, ws, image, on)) != cudaSuccess)
+        if ((e = sg::pt_wave(dev, base, tree, cam, width, height, p0 + from, std::min(part, P - from), key, first,
+                             std::min(per_wave, spp - first), max_depth, ws, image + 3 * (int64_t)from, on)) !=
+            cudaSuccess)
             return pt_fail(e);
     }
     // Every stream's work is done before the scale: the last addition closes

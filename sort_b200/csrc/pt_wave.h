@@ -7,6 +7,8 @@
 
 #include <cstdint>
 
+#include <cstdint>
+
 #include "pt_types.h"
 #include "trace_kernels.h"
 
@@ -22,6 +24,12 @@ constexpr int kInFlight = 2;
 // 0.285 ms, 480x270 at 16 spp from 6.03 to 2.16, a mix of 24 served renders
 // (64x36 to 960x540, 1 to 16 spp) from 28.7 to 12.9.
 constexpr int64_t kWavePaths = int64_t(1) << 20;
+
+// Paths a wave holds at most, and slots of a server's pool (serve_kernels.h): a
+// shadow queue has two rays per path in eight planes, and the kernels find a place
+// in it with an int. Larger frames go in several waves per sample.
+constexpr int64_t kMaxWavePaths = int64_t(1) << 27;
+static_assert(8 * (2 * kMaxWavePaths) - 1 <= INT32_MAX, "a place in the shadow queue's planes is an int");
 
 // Samples per wave of a band of n pixels whose buffers hold cap paths.
 inline int wave_samples(int64_t n, int64_t cap, int spp) {

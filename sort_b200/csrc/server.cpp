@@ -654,11 +654,12 @@ sg_status sg_server_create(const sg_server_opts* opts, sg_server** out) {
     sg_server* S = new (std::nothrow) sg_server;
     if (!S) return fail(SG_ERR_OUT_OF_MEMORY, "host allocation failed");
     S->opts = o;
+    S->opts.path_slots = std::min(o.path_slots, sg::kMaxWavePaths);  // a smaller pool gives the same images
     S->solo_pixels = o.solo_pixels < 0 ? 0 : o.solo_pixels > 0 ? o.solo_pixels : int64_t(1);
     S->arena = Arena(o.pixel_budget);
     S->slot_ticket.assign(size_t(o.max_requests), -1);
     for (int r = o.max_requests - 1; r >= 0; --r) S->free_slots.push_back(r);
-    const size_t C = size_t(o.path_slots), R = size_t(o.max_requests), P = size_t(o.pixel_budget);
+    const size_t C = size_t(S->opts.path_slots), R = size_t(o.max_requests), P = size_t(o.pixel_budget);
     // Device layout.
     sg::SrvBuffers& b = S->b;
     int* st_arrays[5];
