@@ -448,7 +448,7 @@ sg_status pump_lane(sg_server* S, int l) {
                 if (u.submit_ns < t.submit_ns || (u.submit_ns == t.submit_ns && o.id < L.id)) oldest = false;
             }
     }
-    const int rows = std::max(1, L.w[0].cap / q.width);  // rows per band: a band fits the wave buffers
+    const int64_t P = int64_t(q.width) * q.height;
     while (!end && L.next < L.last && L.next - L.done < 2) {
         // Wave k on buffer set and stream pair k % 2; its image additions
         // wait for wave k - 1's.
@@ -459,11 +459,10 @@ sg_status pump_lane(sg_server* S, int l) {
         const int prio = oldest ? 0 : 1;
         const cudaStream_t on = L.stream[prio][k % 2];
         w.side = L.side[prio][k % 2];
-        for (int y = 0; y < q.height && e == cudaSuccess; y += rows) {
-            const int y1 = std::min(q.height, y + rows);
-            const int p0 = y * q.width;
-            e = sg::pt_wave(sc.pt, base, sc.tree, q.cam, q.width, q.height, p0, (y1 - y) * q.width, q.key,
-                            first, samples, q.max_depth, w, q.image + 3 * int64_t(p0), on);
+        for (int64_t p0 = 0; p0 < P && e == cudaSuccess; p0 += w.cap) {  // the pixels that fit the wave buffers
+            e = sg::pt_wave(sc.pt, base, sc.tree, q.cam, q.width, q.height, int(p0),
+                            int(std::min<int64_t>(w.cap, P - p0)), q.key, first, samples, q.max_depth, w,
+                            q.image + 3 * p0, on);
         }
         if (e == cudaSuccess) e = cudaEventRecord(L.wave_done[k % 2], on);
         if (e != cudaSuccess) return fail(SG_ERR_CUDA, std::string("solo wave: ") + cudaGetErrorString(e));

@@ -1,6 +1,7 @@
 """Frames and pools at the size limits: places in a wave's shadow queue (two rays per
 path, eight planes) are ints, so a wave holds at most 2^27 paths and a larger frame
-takes several waves per sample; a server's pool holds no more slots."""
+takes several waves per sample; a server's pool holds no more slots. A request's rows
+may be longer than a server's pool has slots."""
 import numpy as np
 import pytest
 
@@ -44,5 +45,20 @@ def test_largest_pool_renders_the_same_image(tracer):
         sid = srv.add_scene(tracer)
         img, res = srv.wait(srv.submit(sid, scenes.CAMERA, 64, 36, 2, 5, seed=6))
         assert res["status"] == 0 and np.array_equal(img.view(np.int32), want.view(np.int32))
+    finally:
+        srv.close()
+
+
+@pytest.mark.parametrize("spp", [1, 3])
+def test_rows_longer_than_the_pool(tracer, spp):
+    from sort_b200 import scenes
+    from sort_b200.server import RenderServer
+    want = tracer.Render(scenes.CAMERA, 201, 3, spp, 4, seed=7).cpu().numpy()
+    srv = RenderServer(path_slots=64, pixel_budget=1 << 12)
+    try:
+        sid = srv.add_scene(tracer)
+        for _ in range(2):
+            img, res = srv.wait(srv.submit(sid, scenes.CAMERA, 201, 3, spp, 4, seed=7))
+            assert res["status"] == 0 and np.array_equal(img.view(np.int32), want.view(np.int32))
     finally:
         srv.close()
