@@ -466,7 +466,7 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
     int64_t waves;
     size_t cap, scap, need;
     for (;;) {
-        waves = (int64_t)((spp + per_wave - 1) / per_wave) * parts;
+        waves = (int64_t)sg::wave_count(spp, per_wave) * parts;
         in_flight = waves < sg::kInFlight ? (int)waves : sg::kInFlight;
         cap = (size_t)part * per_wave;
         scap = 2 * cap;

@@ -37,6 +37,9 @@ inline int wave_samples(int64_t n, int64_t cap, int spp) {
     return most < 1 ? 1 : (most > spp ? spp : (int)most);
 }
 
+// Waves of `samples` samples each that spp samples take (any int: no sum of the two).
+inline int wave_count(int spp, int samples) { return spp / samples + (spp % samples ? 1 : 0); }
+
 // Queue lengths and ray counters of one bounce; bounce b uses entry b % 4 of the
 // wave's kWaveCounts entries. Shading bounce b appends to entry b + 1 and clears
 // entry b + 2, whose last users (bounce b - 2) are done, so that no memset or

@@ -350,7 +350,7 @@ void start_solo(sg_server* S) {
         L.id = id;
         L.next = L.done = 0;
         L.samples = sg::wave_samples(int64_t(t.req.width) * t.req.height, L.w[0].cap, t.req.spp);
-        L.last = (t.req.spp + L.samples - 1) / L.samples;
+        L.last = sg::wave_count(t.req.spp, L.samples);
         L.finishing = false;
     }
 }
