@@ -179,8 +179,7 @@ struct sg_pt_scene {
     sg::PtLight light{};
     // Per-render buffers, grown on demand.
     int cap = 0;
-    void* d_buf = nullptr;
-    size_t buf_bytes = 0;
+    sg::WaveBuffers buf;
     unsigned long long* d_totals = nullptr;  // rays traced by the last render: extension, shadow
     // kInFlight waves are in flight at once, each with its own buffers:
     // wave k runs on the caller's stream (k % kInFlight == 0) or on
@@ -207,6 +206,16 @@ extern "C" sg_status sg_pt_ray_counts(const sg_pt_scene* ps, int64_t* extension,
 }
 
 namespace {
+
+// The device's memory, as fit_wave_buffers asks for it.
+struct RenderMemory {
+    cudaError_t alloc(size_t bytes, char** mem) const {
+        const cudaError_t e = cudaMalloc(mem, bytes);
+        if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();  // the caller handles it; no launch check may see it
+        return e;
+    }
+    void release(char* mem) const { cudaFree(mem); }
+};
 
 sg_status pt_fail(cudaError_t e) { return sg::set_error(SG_ERR_CUDA, cudaGetErrorString(e)); }
 
@@ -325,7 +334,7 @@ extern "C" sg_status sg_pt_destroy(sg_pt_scene* ps) {
     cudaSetDevice(ps->device);
     if (ps->d_prim) cudaFree(ps->d_prim);
     if (ps->d_mats) cudaFree(ps->d_mats);
-    if (ps->d_buf) cudaFree(ps->d_buf);
+    if (ps->buf.mem) cudaFree(ps->buf.mem);
     for (int k = 0; k < sg::kInFlight; ++k) {
         for (cudaStream_t t : {ps->extra[k], ps->side[k]})
             if (t) {
@@ -455,43 +464,16 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
     } restore{prev};
     cudaStream_t s = (cudaStream_t)stream;
 
-    // Buffers of each wave in flight: two extension queues (rays + slots), hits,
-    // one shadow queue of 2 entries per path (rays + contributions), occlusion
-    // flags, throughput and radiance, shadow entries, counts; then the shared ray
-    // totals.
-    auto align = [](size_t x) { return (x + 255) & ~size_t(255); };
-    // A frame too large for one wave goes in parts of `part` pixels.
-    const int part = (int)std::min<int64_t>(P, sg::kMaxWavePaths), parts = (P + part - 1) / part;
-    int per_wave = sg::wave_samples(P, sg::kWavePaths, spp), in_flight;
-    int64_t waves;
-    size_t cap, scap, need;
-    for (;;) {
-        waves = (int64_t)sg::wave_count(spp, per_wave) * parts;
-        in_flight = waves < sg::kInFlight ? (int)waves : sg::kInFlight;
-        cap = (size_t)part * per_wave;
-        scap = 2 * cap;
-        const size_t qbytes = align(cap * 8 * 4) + align(cap * 4);
-        const size_t set = 2 * qbytes + align(cap * 4) * 2 + align(scap * 8 * 4) + align(scap * 3 * 4) + align(scap) +
-                           align(cap * 6 * 4) + align(cap * 2 * 4) + align(sg::kWaveCounts * sizeof(sg::WaveCount));
-        need = in_flight * set + align(16);
-        if (ps->buf_bytes >= need) break;
-        if (ps->d_buf) cudaFree(ps->d_buf);
-        ps->d_buf = nullptr;
-        ps->d_totals = nullptr;
-        ps->buf_bytes = 0;
-        e = cudaMalloc(&ps->d_buf, need);
-        if (e == cudaSuccess) {
-            ps->buf_bytes = need;
-            break;
-        }
-        if (e != cudaErrorMemoryAllocation || per_wave == 1) return pt_fail(e);
-        (void)cudaGetLastError();  // fewer samples share a wave: less memory, the same image
-        per_wave = (per_wave + 1) / 2;
-    }
-    char* b = (char*)ps->d_buf;
+    ps->d_totals = nullptr;  // until this render's buffers stand
+    sg::WavePlan plan;
+    if ((e = sg::fit_wave_buffers(RenderMemory{}, ps->buf, P, spp, plan)) != cudaSuccess) return pt_fail(e);
+    const int part = plan.part, parts = plan.parts, per_wave = plan.per_wave, in_flight = plan.in_flight;
+    const int64_t waves = plan.waves;
+    const size_t cap = plan.cap, scap = 2 * cap;
+    char* b = ps->buf.mem;
     auto take = [&](size_t bytes) {
         char* r = b;
-        b += align(bytes);
+        b += sg::wave_align(bytes);
         return r;
     };
     bool made = true;
@@ -525,7 +507,7 @@ extern "C" sg_status sg_pt_render_rows(sg_pt_scene* ps, const float* camera, int
         w[k].flush_done = ps->flushed[k];
     }
     unsigned long long* totals = (unsigned long long*)take(16);  // rays traced: extension, shadow
-    if ((size_t)(b - (char*)ps->d_buf) > need) return sg::set_error(SG_ERR_INTERNAL, "render buffer layout overflow");
+    if ((size_t)(b - ps->buf.mem) > plan.bytes) return sg::set_error(SG_ERR_INTERNAL, "render buffer layout overflow");
     for (sg::PtWave& x : w) x.totals = totals;
     ps->d_totals = totals;
     if ((e = cudaMemsetAsync(totals, 0, 16, s)) != cudaSuccess) return pt_fail(e);

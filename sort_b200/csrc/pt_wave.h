@@ -51,6 +51,71 @@ struct WaveCount {
 };
 constexpr int kWaveCounts = 4;
 
+// A render of `pixels` pixels as waves: of `part` pixels (a frame too large for one
+// wave goes in `parts` of them) and per_wave samples each, in_flight at once, each
+// with its own set of buffers.
+struct WavePlan {
+    int part, parts, per_wave, in_flight;
+    int64_t waves;
+    size_t cap;    // paths of a set
+    size_t bytes;  // of every set, and the ray totals
+};
+inline size_t wave_align(size_t x) { return (x + 255) & ~size_t(255); }
+inline WavePlan wave_plan(int64_t pixels, int spp, int per_wave) {
+    WavePlan w;
+    w.part = (int)(pixels < kMaxWavePaths ? pixels : kMaxWavePaths);
+    w.parts = (int)((pixels + w.part - 1) / w.part);
+    w.per_wave = per_wave;
+    w.waves = (int64_t)wave_count(spp, per_wave) * w.parts;
+    w.in_flight = w.waves < kInFlight ? (int)w.waves : kInFlight;
+    w.cap = (size_t)w.part * per_wave;
+    const size_t cap = w.cap, scap = 2 * cap;
+    // two extension queues (rays, paths), hits, the shadow queue (rays,
+    // contributions), occlusion flags, throughput and radiance, shadow entries, counts
+    const size_t set = 2 * (wave_align(cap * 32) + wave_align(cap * 4)) + 2 * wave_align(cap * 4) +
+                       wave_align(scap * 32) + wave_align(scap * 12) + wave_align(scap) + wave_align(cap * 24) +
+                       wave_align(cap * 8) + wave_align(kWaveCounts * sizeof(WaveCount));
+    w.bytes = w.in_flight * set + wave_align(16);
+    return w;
+}
+
+// The memory a scene's renders keep between them.
+struct WaveBuffers {
+    char* mem = nullptr;
+    size_t bytes = 0;
+    size_t most = SIZE_MAX;  // what samples sharing waves may take: less than what could not be had once
+};
+
+// Makes `buf` large enough for a render and says how it goes. Samples share waves by
+// fewer where the memory cannot be had; the next render does not ask for it again, and
+// the memory held is given up only for more, or where not even a sample per wave fits it.
+// Gpu: cudaError_t alloc(bytes, &mem), release(mem).
+template <class Gpu>
+cudaError_t fit_wave_buffers(Gpu&& gpu, WaveBuffers& buf, int64_t pixels, int spp, WavePlan& plan) {
+    for (int per_wave = wave_samples(pixels, kWavePaths, spp);; per_wave = (per_wave + 1) / 2) {
+        plan = wave_plan(pixels, spp, per_wave);
+        if (plan.bytes <= buf.bytes) return cudaSuccess;
+        char* mem = nullptr;
+        if (per_wave == 1) {
+            if (buf.mem) gpu.release(buf.mem);
+            buf.mem = nullptr;
+            buf.bytes = 0;
+            const cudaError_t e = gpu.alloc(plan.bytes, &mem);
+            if (e != cudaSuccess) return e;
+        } else {
+            if (plan.bytes > buf.most) continue;
+            if (gpu.alloc(plan.bytes, &mem) != cudaSuccess) {
+                buf.most = plan.bytes - 1;
+                continue;
+            }
+            if (buf.mem) gpu.release(buf.mem);
+        }
+        buf.mem = mem;
+        buf.bytes = plan.bytes;
+        return cudaSuccess;
+    }
+}
+
 // Device buffers of a wave: two extension queues (8 floats per ray with stride
 // cap, a path index per entry), the hits (cap each), the shadow queue (stride
 // 2 * cap, three contribution planes) and its occlusion flags, per-path
