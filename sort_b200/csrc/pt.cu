@@ -209,6 +209,10 @@ namespace {
 
 // The device's memory, as fit_wave_buffers asks for it.
 struct RenderMemory {
+    size_t free_bytes() const {
+        size_t free = 0, total = 0;
+        return cudaMemGetInfo(&free, &total) == cudaSuccess ? free : 0;
+    }
     cudaError_t alloc(size_t bytes, char** mem) const {
         const cudaError_t e = cudaMalloc(mem, bytes);
         if (e == cudaErrorMemoryAllocation) (void)cudaGetLastError();  // the caller handles it; no launch check may see it

@@ -86,10 +86,12 @@ struct WaveBuffers {
     size_t most = SIZE_MAX;  // what samples sharing waves may take: less than what could not be had once
 };
 
-// Makes `buf` large enough for a render and says how it goes. Samples share waves by
-// fewer where the memory cannot be had; the next render does not ask for it again, and
-// the memory held is given up only for more, or where not even a sample per wave fits it.
-// Gpu: cudaError_t alloc(bytes, &mem), release(mem).
+// Makes `buf` large enough for a render and says how it goes. Samples that share waves
+// take up to 424 MB where a sample per wave takes 404 bytes per pixel, so they get a
+// sixteenth of the device's free memory at most and share by fewer where that, or
+// what can be had, is less; the next render does not ask for it again, and the
+// memory held is given up only for more, or where not even a sample per wave fits it.
+// Gpu: size_t free_bytes(), cudaError_t alloc(bytes, &mem), release(mem).
 template <class Gpu>
 cudaError_t fit_wave_buffers(Gpu&& gpu, WaveBuffers& buf, int64_t pixels, int spp, WavePlan& plan) {
     for (int per_wave = wave_samples(pixels, kWavePaths, spp);; per_wave = (per_wave + 1) / 2) {
@@ -104,7 +106,7 @@ cudaError_t fit_wave_buffers(Gpu&& gpu, WaveBuffers& buf, int64_t pixels, int sp
             if (e != cudaSuccess) return e;
         } else {
             if (plan.bytes > buf.most) continue;
-            if (gpu.alloc(plan.bytes, &mem) != cudaSuccess) {
+            if (plan.bytes > gpu.free_bytes() / 16 || gpu.alloc(plan.bytes, &mem) != cudaSuccess) {
                 buf.most = plan.bytes - 1;
                 continue;
             }

@@ -41,8 +41,9 @@ int main() {
 
 
 def test_memory_of_waves(tmp_path):
-    """A size that could not be had is not asked for again by the next render, and what
-    a scene holds is released only for something larger, or to make room for a sample
+    """Samples that share waves take no more than a sixteenth of the free memory, a
+    size that could not be had is not asked for again by the next render, and what a
+    scene holds is released only for something larger, or to make room for a sample
     per wave."""
     run(tmp_path, """
 struct Fake {
@@ -51,6 +52,7 @@ struct Fake {
     cudaError_t error = cudaErrorMemoryAllocation;
     std::vector<size_t> asked, live;
     int released = 0;
+    size_t free_bytes() const { return free; }
     cudaError_t alloc(size_t bytes, char** mem) {
         asked.push_back(bytes);
         if (bytes > free || bytes > limit) return error;
@@ -81,6 +83,17 @@ int main() {
         CHECK(b.bytes == p.bytes && g.asked.size() == 1);
         CHECK(fit_wave_buffers(g, b, 64 * 64, 4096, p) == cudaSuccess && p.per_wave == 256);
         CHECK(fit_wave_buffers(g, b, 61, 4096, p) == cudaSuccess && g.asked.size() == 1 && g.released == 0);
+    }
+    {  // little room: at most a sixteenth of it, and no attempt at more
+        Fake g;
+        g.free = 2 * GiB;
+        WaveBuffers b;
+        CHECK(fit_wave_buffers(g, b, 64 * 64, 4096, p) == cudaSuccess);
+        CHECK(p.per_wave > 1 && b.bytes <= 128 * MiB && g.asked.size() == 1);
+        const size_t held = b.bytes;
+        g.free = 170 * GiB;
+        CHECK(fit_wave_buffers(g, b, 64 * 64, 4096, p) == cudaSuccess);
+        CHECK(b.bytes == held && g.asked.size() == 1 && g.released == 0);
     }
     {  // allocations fail above 100 MiB: fewer samples share a wave, remembered by the next renders
         Fake g;
