@@ -178,7 +178,6 @@ struct sg_pt_scene {
     sg::PtMaterial* d_mats = nullptr;
     sg::PtLight light{};
     // Per-render buffers, grown on demand.
-    int cap = 0;
     sg::WaveBuffers buf;
     unsigned long long* d_totals = nullptr;  // rays traced by the last render: extension, shadow
     // kInFlight waves are in flight at once, each with its own buffers:

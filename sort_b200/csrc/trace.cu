@@ -35,17 +35,15 @@
 
 namespace sg {
 
-// The counting launches' kernel: one ray per thread (`Traversal`). With n_dev set, the
-// batch size is min(n, *n_dev), read on the device. Q8 reads 8-bit nodes.
+// The counting launches' kernel: one ray per thread (`Traversal`). Q8 reads 8-bit nodes.
 template <int W, bool ANY, int STACK, bool Q8>
 __global__ void __launch_bounds__(128, 9) k_trace_stats(DevTree tr, DevRays rays, int64_t n,
                                                         int32_t* __restrict__ prim_out, float* __restrict__ t_out,
                                                         float* __restrict__ u_out, float* __restrict__ v_out,
                                                         uint8_t* __restrict__ occ_out, int* __restrict__ err,
-                                                        unsigned long long* __restrict__ stats,
-                                                        const int* __restrict__ n_dev) {
+                                                        unsigned long long* __restrict__ stats) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if ((n_dev && i >= (int64_t)*n_dev) || i >= n) return;
+    if (i >= n) return;
     Traversal<W, ANY, STACK, true, Q8, true> tv;
     uint2 stk_mem[STACK];
     tv.stk = stk_mem;
@@ -57,7 +55,8 @@ __global__ void __launch_bounds__(128, 9) k_trace_stats(DevTree tr, DevRays rays
 
 // Launch shape of k_trace_walk per tree form: blocks of 128 per SM (registers:
 // 72 at 7 blocks hold the width-8 FP32 walk without a spill, 64 at 8 blocks the
-// others) and the idle lanes at which a warp takes new rays. Measured, same
+// others, but for 20 bytes of the 8-bit any-hit walk) and the idle lanes at which a
+// warp takes new rays. Measured, same
 // box, width 8: 7 blocks 2.54 / 2.10 ms on 4M diffuse / shadow rays (21M
 // triangles), 8 blocks (88 bytes spilled) 2.98 / 2.25, 9 blocks 2.96 / 2.40.
 // 8-bit nodes: 0.338 / 0.334 / 0.336 ms at 7 / 8 / 9 blocks on 700k rays.
@@ -95,17 +94,11 @@ struct TraceJob {
     float* v_out;
     uint8_t* occ_out;
     unsigned* counter;
-    int n, span, step;  // step: rays between a warp's spans
-    int next, end;
+    int n;
+    int next, end;  // rays left: the warp's span, or, with a counter, all of them until it has passed n
 
     __device__ __forceinline__ const DevTree& tree() const { return tr; }
-    __device__ __forceinline__ bool more() {
-        if (next < end) return true;
-        if (counter || end >= n - (step - span)) return false;
-        next = end + (step - span);
-        end = n - next < span ? n : next + span;
-        return true;
-    }
+    __device__ __forceinline__ bool more() const { return next < end; }
     __device__ __forceinline__ bool take(bool idle, unsigned mask, int lane, WalkShared* sh, RayState& r,
                                          const DevTree&) {
         if (counter) {
@@ -168,11 +161,10 @@ __global__ void __launch_bounds__(kWalkThreads, WalkShape<W, Q8>::kBlocks)
         span = (n + slots - 1) / slots;
         counter = nullptr;
     }
-    TraceJob job{tr, rays, order, prim_out, t_out, u_out, v_out, ANY ? occ_out : nullptr, counter, n, span, 0, 0, n};
+    TraceJob job{tr, rays, order, prim_out, t_out, u_out, v_out, ANY ? occ_out : nullptr, counter, n, 0, n};
     if (!counter) {
         const int64_t first = (int64_t)warp * span;
         if (first >= n) return;
-        job.step = (int)gridDim.x * kWalkWarps * span;
         job.next = (int)first;
         job.end = n - job.next < span ? n : job.next + span;
     }
@@ -283,7 +275,9 @@ static cudaError_t launch_walk(const TraceLaunch& L, const DevTree& tr, const De
     // memory for one the launch goes by spans, as those do: 2.68 against 2.15 ms
     // on 4M diffuse rays.
     char* scratch = nullptr;
-    if (!counter && L.scratch && !L.n_dev && n > (int64_t)slots * 32) {
+    if (L.n_dev && (n > kMaxWalkRays || (!counter && n > (int64_t)slots * 32)))
+        return cudaErrorInvalidValue;  // one launch, and its length is known on the device alone
+    if (!counter && L.scratch && n > (int64_t)slots * 32) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) {
             (void)cudaGetLastError();
@@ -304,7 +298,7 @@ static cudaError_t launch_walk(const TraceLaunch& L, const DevTree& tr, const De
         int64_t warps = slots;
         if (m <= slots * 32)
             warps = m < slots ? m : slots;
-        else if (!counter && !L.n_dev)
+        else if (!counter)
             warps = (m + kWalkSpan - 1) / kWalkSpan;
         if (scratch && (e = cudaMemsetAsync(counter, 0, sizeof(unsigned), s)) != cudaSuccess) break;
         const DevRays r{rays.ox + a, rays.oy + a, rays.oz + a,   rays.dx + a,
@@ -445,10 +439,10 @@ static cudaError_t launch_stack(const TraceLaunch& L, const DevTree& tr, const D
         const unsigned blocks = (unsigned)((n + 127) / 128);
         if (L.q8)
             k_trace_stats<W, ANY, STACK, true><<<blocks, 128, 0, s>>>(tr, rays, n, L.prim, L.t, L.u, L.v, L.occ, L.err,
-                                                                      L.stats, L.n_dev);
+                                                                      L.stats);
         else
             k_trace_stats<W, ANY, STACK, false><<<blocks, 128, 0, s>>>(tr, rays, n, L.prim, L.t, L.u, L.v, L.occ, L.err,
-                                                                       L.stats, L.n_dev);
+                                                                       L.stats);
         return cudaGetLastError();
     }
     // The automatic choice is batch order at every size: with lanes refilled and

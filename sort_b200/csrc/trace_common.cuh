@@ -89,46 +89,22 @@ __device__ __forceinline__ float root_intersect(const RayState& r, const float* 
 // slab interval is non-empty; d gets fmin on a hit and -1 on a miss, as SORT's
 // simd_pick_ps leaves it (validity of the slot is checked by the caller).
 //
+// SORT takes t(lo) = -o/d + lo * 1/d and t(hi) per axis and their minimum and
+// maximum; here n is the axis's entry plane and f its exit plane (n = lo, f = hi
+// where 1/d > 0, swapped where 1/d < 0). With 1/d finite and non-zero and
+// lo <= hi, t(b) = fl(-o/d + fl(b * 1/d)) is monotonic in b, so t(n) =
+// min(t(lo), t(hi)) and t(f) = max(...) exactly, and the interval's bounds are the
+// same maxima and minima in another order: the result equals SORT's for every box
+// with lo <= hi. Only empty slots (lo = +FLT_MAX > hi = -FLT_MAX) differ, and the
+// caller discards those by their -1 reference. That is two flops and two
+// comparisons fewer per axis.
+//
 // SORT's lanes use _mm_min_ps / _mm_max_ps (a < b ? a : b); here fminf / fmaxf,
 // one instruction each. The two agree in value whenever neither input is NaN,
 // and no input is: 1/d and -o/d are finite after the |d| >= 1e-5 clamp, box
 // bounds are finite or +-FLT_MAX, so every t is finite or +-inf (rays must be
 // finite, as SORT assumes). Where they may differ — which of +0 and -0 an equal
 // pair returns — nothing downstream looks: entry distances are only compared.
-__device__ __forceinline__ bool slab(const RayState& r, float lx, float hx, float ly, float hy, float lz, float hz,
-                                     float& d) {
-    float f_min = r.tmin, f_max = r.tmax;
-    {
-        const float t1 = __fadd_rn(r.od[0], __fmul_rn(r.rcp[0], hx));
-        const float t2 = __fadd_rn(r.od[0], __fmul_rn(r.rcp[0], lx));
-        f_min = fmaxf(f_min, fminf(t1, t2));
-        f_max = fminf(f_max, fmaxf(t1, t2));
-    }
-    {
-        const float t1 = __fadd_rn(r.od[1], __fmul_rn(r.rcp[1], hy));
-        const float t2 = __fadd_rn(r.od[1], __fmul_rn(r.rcp[1], ly));
-        f_min = fmaxf(f_min, fminf(t1, t2));
-        f_max = fminf(f_max, fmaxf(t1, t2));
-    }
-    {
-        const float t1 = __fadd_rn(r.od[2], __fmul_rn(r.rcp[2], hz));
-        const float t2 = __fadd_rn(r.od[2], __fmul_rn(r.rcp[2], lz));
-        f_min = fmaxf(f_min, fminf(t1, t2));
-        f_max = fminf(f_max, fmaxf(t1, t2));
-    }
-    const bool hit = f_min <= f_max;
-    d = hit ? f_min : -1.0f;
-    return hit;
-}
-
-// slab() from each axis's entry plane n and exit plane f (n = lo, f = hi where
-// 1/d > 0, swapped where 1/d < 0). With 1/d finite and non-zero and lo <= hi,
-// t(b) = fl(-o/d + fl(b * 1/d)) is monotonic in b, so t(n) = min(t(lo), t(hi))
-// and t(f) = max(...) exactly, and the interval's bounds are the same maxima and
-// minima in another order: the result equals slab()'s for every box with
-// lo <= hi. Only empty slots (lo = +FLT_MAX > hi = -FLT_MAX) differ, and the
-// caller discards those by their -1 reference. Two flops and two comparisons
-// fewer per axis.
 __device__ __forceinline__ bool slab_near_far(const RayState& r, float nx, float fx, float ny, float fy, float nz,
                                               float fz, float& d) {
     const float tnx = __fadd_rn(r.od[0], __fmul_rn(r.rcp[0], nx));

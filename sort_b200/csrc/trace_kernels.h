@@ -35,7 +35,7 @@ struct TraceLaunch {
     unsigned long long* stats = nullptr;  // non-null: also accumulate SORT's traversal counters
     unsigned* counter = nullptr;  // zero when the launch starts: warps take rays from it (null: the launch finds its own)
     bool scratch = true;          // the launch may take stream-ordered scratch from the library's pool
-    const int* n_dev = nullptr;   // if set, the batch is min(n, *n_dev); large ones want a counter
+    const int* n_dev = nullptr;   // if set, the batch is min(n, *n_dev), n <= 2^30; needs a counter (not in counting launches)
     bool q8 = false;             // interior nodes in the 8-bit format
 };
 

@@ -129,9 +129,8 @@ __device__ __forceinline__ void load_node_q8(const float4* __restrict__ nodes, i
 // distance the negative of that), so only a ray with a NaN or infinite
 // component can reach one. An empty 8-bit slot decodes to an inverted box
 // (lower bound 255 steps above the upper one), which such a ray misses too.
-// Dropping the per-child test saves two instructions per child and six
-// registers in the closest-hit kernel; skipping in step() keeps any empty
-// entry that is reached harmless.
+// Dropping the per-child test saves two instructions per child; skipping in
+// step() keeps any empty entry that is reached harmless.
 template <int W, bool ANY, int STACK, bool STATS, bool Q8 = false, bool STEP_SKIPS_EMPTY = false>
 struct Traversal {
     static constexpr bool kTestEmpty = !STEP_SKIPS_EMPTY;
@@ -278,26 +277,6 @@ struct Traversal {
         }
         const int cnt = __popc(mask);
         if (cnt == 0) return false;
-        if (ANY && !STATS) {
-            // Any hit: before the first hit nothing is culled (the current hit
-            // distance stays FLT_MAX), so the answer is whether any triangle of
-            // the nodes the slab tests reach is hit, whatever the visit order.
-            // Descend into the lowest hit slot, push the others; SORT's
-            // near-first order is kept only where its counts are wanted.
-            const unsigned first = mask & (0u - mask);  // lowest set bit
-            int32_t fc = 0;
-#pragma unroll
-            for (int j = 0; j < W; ++j) {
-                if (!(mask & (1u << j))) continue;
-                if ((1u << j) == first)
-                    fc = nd.ch[j];
-                else
-                    stk[si++] = make_uint2((uint32_t)nd.ch[j], 0u);  // entry distance 0: never culled
-            }
-            cur = fc;
-            cur_d = 0.0f;
-            return true;
-        }
         if (cnt == 1) {
 #pragma unroll
             for (int j = 0; j < W; ++j)
