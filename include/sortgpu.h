@@ -486,9 +486,9 @@ sg_status sg_batcher_autotune(sg_batcher* batcher, const sg_batch* batches, cons
  *   max_recursive_depth; ordered on `stream`. The scene keeps the memory of its
  *   largest render until it is destroyed: 404 bytes per pixel (202 at 1 spp; at
  *   most 54 GB, for frames of 2^27 pixels and more). A frame of fewer than 2^20
- *   pixels renders several samples at a time where that takes no more than a
- *   sixteenth of the device's free memory: up to 424 MB. Less memory gives the same
- *   image. */
+ *   pixels renders several samples at a time where that takes no more than 64 MB
+ *   or a sixteenth of the device's free memory: up to 424 MB. Less memory gives the
+ *   same image. */
 typedef struct sg_pt_scene sg_pt_scene;
 sg_status sg_pt_create(const sg_scene* scene, const float* triangles, int64_t ntri, const int32_t* mat_of_tri,
                        const float* materials, int32_t nmat, const float* light, sg_pt_scene** out);

@@ -87,11 +87,13 @@ struct WaveBuffers {
 };
 
 // Makes `buf` large enough for a render and says how it goes. Samples that share waves
-// take up to 424 MB where a sample per wave takes 404 bytes per pixel, so they get a
-// sixteenth of the device's free memory at most and share by fewer where that, or
-// what can be had, is less; the next render does not ask for it again, and the
-// memory held is given up only for more, or where not even a sample per wave fits it.
+// take up to 424 MB where a sample per wave takes 404 bytes per pixel, so beyond
+// kAskBytes they get a sixteenth of the device's free memory at most and share by
+// fewer where that, or what can be had, is less; the next render does not ask for it
+// again, and the memory held is given up only for more, or where not even a sample per
+// wave fits it. (Asking takes 70 to 100 us, a tenth of a small scene's first render.)
 // Gpu: size_t free_bytes(), cudaError_t alloc(bytes, &mem), release(mem).
+constexpr size_t kAskBytes = size_t(64) << 20;
 template <class Gpu>
 cudaError_t fit_wave_buffers(Gpu&& gpu, WaveBuffers& buf, int64_t pixels, int spp, WavePlan& plan) {
     for (int per_wave = wave_samples(pixels, kWavePaths, spp);; per_wave = (per_wave + 1) / 2) {
@@ -106,7 +108,8 @@ cudaError_t fit_wave_buffers(Gpu&& gpu, WaveBuffers& buf, int64_t pixels, int sp
             if (e != cudaSuccess) return e;
         } else {
             if (plan.bytes > buf.most) continue;
-            if (plan.bytes > gpu.free_bytes() / 16 || gpu.alloc(plan.bytes, &mem) != cudaSuccess) {
+            if ((plan.bytes > kAskBytes && plan.bytes > gpu.free_bytes() / 16) ||
+                gpu.alloc(plan.bytes, &mem) != cudaSuccess) {
                 buf.most = plan.bytes - 1;
                 continue;
             }

@@ -41,8 +41,8 @@ int main() {
 
 
 def test_memory_of_waves(tmp_path):
-    """Samples that share waves take no more than a sixteenth of the free memory, a
-    size that could not be had is not asked for again by the next render, and what a
+    """Samples that share waves take no more than 64 MB or a sixteenth of the free memory
+    (asked for above 64 MB only), a size that could not be had is not asked for again by the next render, and what a
     scene holds is released only for something larger, or to make room for a sample
     per wave."""
     run(tmp_path, """
@@ -52,7 +52,8 @@ struct Fake {
     cudaError_t error = cudaErrorMemoryAllocation;
     std::vector<size_t> asked, live;
     int released = 0;
-    size_t free_bytes() const { return free; }
+    int asked_free = 0;
+    size_t free_bytes() { ++asked_free; return free; }
     cudaError_t alloc(size_t bytes, char** mem) {
         asked.push_back(bytes);
         if (bytes > free || bytes > limit) return error;
@@ -83,6 +84,11 @@ int main() {
         CHECK(b.bytes == p.bytes && g.asked.size() == 1);
         CHECK(fit_wave_buffers(g, b, 64 * 64, 4096, p) == cudaSuccess && p.per_wave == 256);
         CHECK(fit_wave_buffers(g, b, 61, 4096, p) == cudaSuccess && g.asked.size() == 1 && g.released == 0);
+        CHECK(g.asked_free == 1);
+        WaveBuffers c;  // a small one is not worth asking
+        g.free = 100 * MiB;
+        CHECK(fit_wave_buffers(g, c, 161 * 91, 4, p) == cudaSuccess && p.per_wave == 4 && g.asked_free == 1);
+        CHECK(fit_wave_buffers(g, c, 64 * 64, 4096, p) == cudaSuccess && c.bytes <= 64 * MiB && c.bytes > 32 * MiB);
     }
     {  // little room: at most a sixteenth of it, and no attempt at more
         Fake g;
