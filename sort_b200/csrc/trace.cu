@@ -55,8 +55,8 @@ __global__ void __launch_bounds__(128, 9) k_trace_stats(DevTree tr, DevRays rays
 
 // Launch shape of k_trace_walk per tree form: blocks of 128 per SM (registers:
 // 72 at 7 blocks hold the width-8 FP32 walk without a spill, 64 at 8 blocks the
-// others, but for 20 bytes of the 8-bit any-hit walk) and the idle lanes at which a
-// warp takes new rays. Measured, same
+// others but width 8 with 8-bit nodes, 12 bytes) and the idle lanes at which a warp
+// takes new rays. Measured, same
 // box, width 8: 7 blocks 2.54 / 2.10 ms on 4M diffuse / shadow rays (21M
 // triangles), 8 blocks (88 bytes spilled) 2.98 / 2.25, 9 blocks 2.96 / 2.40.
 // 8-bit nodes: 0.338 / 0.334 / 0.336 ms at 7 / 8 / 9 blocks on 700k rays.
@@ -94,7 +94,6 @@ struct TraceJob {
     float* v_out;
     uint8_t* occ_out;
     unsigned* counter;
-    int n;
     int next, end;  // rays left: the warp's span, or, with a counter, all of them until it has passed n
 
     __device__ __forceinline__ const DevTree& tree() const { return tr; }
@@ -105,7 +104,7 @@ struct TraceJob {
             unsigned b = 0;
             if (lane == 0) b = atomicAdd(counter, (unsigned)__popc(mask));
             b = __shfl_sync(kFullWarp, b, 0);
-            next = b < (unsigned)n ? (int)b : n;
+            next = b < (unsigned)end ? (int)b : end;
         }
         const int k = next + __popc(mask & ((1u << lane) - 1u));
         const bool got = idle && k < end;
@@ -161,7 +160,7 @@ __global__ void __launch_bounds__(kWalkThreads, WalkShape<W, Q8>::kBlocks)
         span = (n + slots - 1) / slots;
         counter = nullptr;
     }
-    TraceJob job{tr, rays, order, prim_out, t_out, u_out, v_out, ANY ? occ_out : nullptr, counter, n, 0, n};
+    TraceJob job{tr, rays, order, prim_out, t_out, u_out, v_out, ANY ? occ_out : nullptr, counter, 0, n};
     if (!counter) {
         const int64_t first = (int64_t)warp * span;
         if (first >= n) return;
