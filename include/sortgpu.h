@@ -430,8 +430,9 @@ sg_status sg_trace_closest_host_static(const sg_scene* scene, const float* rays8
  *   > 0 stops warps from claiming rays once that long has passed since the
  *   run's start; the rays they hold still finish. Up to max_batches batches.
  * sg_batcher_wait: synchronises `stream`; per batch of the LAST run (caller
- *   order) the ns from the run's start to the completion of its last ray, or
- *   -1 if the budget left it incomplete (then returns SG_ERR_LIMIT).
+ *   order) the ns from the run's start until its last answer is written (a
+ *   finished ray's answer waits for its warp's next refill, at refill_threshold
+ *   idle lanes or the end of the run), or -1 if the budget left it incomplete (then returns SG_ERR_LIMIT).
  * sg_batcher_autotune: picks, by timing runs of `batches` on `stream`, the
  *   tree width per scene (alternatives[i]: the same triangles built at the
  *   other width, or NULL; use_alternative[i] = 1 where that one is faster) and
@@ -523,7 +524,8 @@ sg_status sg_pt_ray_counts(const sg_pt_scene* pt, int64_t* extension, int64_t* s
  * (work/image_evaluation/image_evaluation.cpp:120-305).
  *
  * sg_server_opts: path_slots = paths in flight (each holds about 250 bytes of
- *   path state in HBM); pixel_budget = pixels of admitted, unfinished requests
+ *   path state in HBM, and about 400 in each of the two solo lanes; 2^27 are used at
+ *   most); pixel_budget = pixels of admitted, unfinished requests
  *   (20 bytes each: image + work queue entry); max_requests = requests admitted
  *   at once; steps_per_poll = bounce steps per graph replay (even, >= 2);
  *   samples_per_claim = samples a pool slot renders of one pixel before the
@@ -531,8 +533,8 @@ sg_status sg_pt_ray_counts(const sg_pt_scene* pt, int64_t* extension, int64_t* s
  *   requests; larger keeps neighbouring pixels together in the queues);
  *   solo_pixels = requests of at least this many pixels and 2 or more
  *   samples take one of the server's solo lanes, in queue order: rendered as
- *   sg_pt_render renders, one wave per sample (two in flight) on the lane's
- *   own buffers, beside the pool, the oldest lane's waves at the highest
+ *   sg_pt_render renders, in waves of one or, for small frames, more samples
+ *   (two in flight) on the lane's own buffers, beside the pool, the oldest lane's waves at the highest
  *   stream priority; the lane scales and completes the request (the image
  *   is the same either way). The pool renders the other requests.
  *   0 = 1 (every multi-sample request), < 0 = never.

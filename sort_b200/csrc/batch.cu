@@ -12,8 +12,10 @@
 //
 // Finished rays are written and counted against their batch when their warp
 // refills (one atomic per batch and refill); the warp that counts a batch's
-// last ray stamps the batch's completion time. A run may carry a time budget: once it has passed, warps
-// stop claiming rays, finish the ones they hold and the run reports the cut.
+// last ray stamps the batch's completion time, which is thus the time its answers
+// are written: a finished ray's wait for its warp's next refill is part of it. A
+// run may carry a time budget: once it has passed, warps stop claiming rays, finish
+// the ones they hold and the run reports the cut.
 #include <cuda_runtime.h>
 
 #include "batch_kernels.h"
@@ -45,7 +47,7 @@ __device__ __forceinline__ int find_batch(const BatchDesc* __restrict__ bt, int 
     return lo;
 }
 
-// Counts the lanes that finished a ray this step against their batches.
+// Counts the lanes whose answers were just written against their batches.
 __device__ __forceinline__ void count_finished(bool fin, int b, const BatchArgs& a, int first, unsigned lane) {
     const unsigned fm = __ballot_sync(0xffffffffu, fin);
     if (fm == 0) return;
@@ -134,9 +136,11 @@ struct BatchJob {
     }
 };
 
-// Held to 896 resident threads per SM (72 registers), as k_trace_walk. 24 batches
-// of 4k .. 1M rays over five scenes (10k .. 2M triangles, width 8): 2.22 -> 1.01
-// ms against one ray per lane with every ray written and counted as it ended.
+// Blocks of 64 and 128: 896 resident threads per SM (72 registers), as k_trace_walk
+// (20 bytes of the 8-bit width-8 walk spill); blocks of 256: three per SM, 768
+// threads (80 registers). 24 batches of 4k .. 1M rays over five scenes (10k .. 2M
+// triangles, width 8) take 1.01 ms; one ray per lane with every ray written and
+// counted as it ends, 2.22.
 template <int W, bool ANY, int STACK, int BLOCK, bool Q8>
 __global__ void __launch_bounds__(BLOCK, 896 / BLOCK) k_trace_batches(const __grid_constant__ BatchArgs a) {
     __shared__ BatchShared shared[BLOCK / 32];

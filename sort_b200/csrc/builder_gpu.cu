@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(256) k_bin(int64_t n, const int* __restrict__ 
     if (one) {  // every thread of the block is in range r (binned or not, uniformly)
         // Straight to the block's bins: a warp's lanes meet four or five deep in
         // a bin, which costs less than grouping them (match, and six reductions
-        // per group): 71 us a round of 5.2M grouped, 56 now.
+        // per group): 56 us a round of 5.2M against 71 grouped.
         if (binned) {
             atomicAdd(&scnt[b], 1u);
             atomic_box(sbox[b], v);
@@ -446,8 +446,8 @@ __device__ __forceinline__ unsigned long long misplaced(int64_t i, int r, const 
 // (left and right in one word), the tiles' prefix sums, then every misplaced
 // element to its place in its list. A range's two counts are equal, so it owns
 // the same places [pair_first, pair_end) in both lists, left ones in order, right
-// ones in order too (k_swap reads them from the end). Flags, two prefix sums and
-// a pairing pass over the primitives took 112 us a round of 5.2M, these take 53.
+// ones in order too (k_swap reads them from the end). 53 us a round of 5.2M; as
+// flags, two prefix sums and a pairing pass over the primitives, 112.
 constexpr int kPairItems = 8, kPairThreads = 512, kPairTile = kPairItems * kPairThreads;
 __global__ void __launch_bounds__(kPairThreads) k_pair_sums(int64_t n, const int* __restrict__ rid,
                                                             const float* __restrict__ cx, const float* __restrict__ cy,
@@ -613,7 +613,8 @@ struct DShape {
 // A node of at most kSmall primitives, split by one warp (k_split_small).
 // Large nodes go through the rounds, whose passes over every primitive cost the
 // same however few are still being split: without small nodes a 5.2M-triangle
-// tree took 72 rounds of 0.45 ms, most of them for ranges of a few hundred.
+// tree takes 72 rounds in place of 48, most of the 24 for ranges of a few hundred.
+// Build of that tree at 256 / 512 / 1,024 / 2,048: 32.6 / 28.1 / 28.1 / 27.1-33 ms.
 constexpr int kSmall = 1024;
 struct SmallNode {
     int32_t id, depth;
@@ -1349,8 +1350,8 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
     // nodes takes its nodes and records from the device (its topology export
     // reads them back from there).
     const bool host = p.host_boxes || p.nextra > 0;
-    // The nodes' numbers (build_tree's, see k_count_inner): on the host this took
-    // 10 ms for 5.2M triangles beside 2 ms of copies.
+    // The nodes' numbers (build_tree's, see k_count_inner): found on the host they
+    // take 10 ms for 5.2M triangles beside 2 ms of copies.
     DevBuf<int32_t> d_inner, d_number, d_base, d_map;
     size_t interior_total = 0;
     if (root_node) {

@@ -91,10 +91,11 @@ struct DevBuf {
 
 // The counts and boxes that a build reads between its kernels land in plain host
 // variables: each is read right after its copy, and a copy to pageable memory
-// returns when it is done. Page-locked words cost more than they gave: a process
-// that holds no other page-locked memory maps and unmaps it with each
-// cudaMallocHost and cudaFreeHost pair, 3.1 ms for the pairs of a build (build and
-// first trace: 1M triangles, Morton tree, 8.3 -> 5.4 ms; 5.2M, SAH, 24.0 -> 20.9).
+// returns when it is done. Page-locked words, two blocks made and freed per build,
+// cost more than they give: build and first trace in processes that do nothing else,
+// medians of 38 and 14 builds in four processes each, 1.3M triangles, Morton tree,
+// 7.8-8.5 ms with page-locked words against 5.2-5.3; 5.2M, SAH, 23.6-25.6 against
+// 20.4-20.8. In a process with render servers the two are level.
 
 inline unsigned grid(int64_t n, int t = 256) { return (unsigned)std::max<int64_t>(1, (n + t - 1) / t); }
 

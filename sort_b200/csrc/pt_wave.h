@@ -19,10 +19,10 @@ constexpr int kInFlight = 2;
 
 // Paths a wave of several samples holds at most: a small frame's samples share
 // waves, because a wave of few paths is bound by its chain of dependent launches
-// and by the latency of single rays, not by the work. A 161x91 frame of 4 spp
-// (four waves of 14,651 paths, then one of 58,604) went from 0.67 to
-// 0.285 ms, 480x270 at 16 spp from 6.03 to 2.16, a mix of 24 served renders
-// (64x36 to 960x540, 1 to 16 spp) from 28.7 to 12.9.
+// and by the latency of single rays, not by the work. One sample per wave against
+// several: a 161x91 frame of 4 spp (four waves of 14,651 paths, or one of 58,604)
+// 0.67 / 0.285 ms, 480x270 at 16 spp 6.03 / 2.16, a mix of 24 served renders
+// (64x36 to 960x540, 1 to 16 spp) 28.7 / 12.9.
 constexpr int64_t kWavePaths = int64_t(1) << 20;
 
 // Paths a wave holds at most, and slots of a server's pool (serve_kernels.h): a

@@ -8,9 +8,9 @@
 //
 // What bounds it and why it has this form. A ray visits about 13.7 nodes and
 // 3.3 leaves of 5.8 triangles (21M triangles, OBVH, diffuse rays), and with one
-// ray per lane from start to end the lanes of a warp part ways: the previous
-// walk kept 14 lanes busy in a node visit, 5 in a leaf, ran a leaf as long as its
-// largest, and issued 26.0k warp instructions per 32 rays at 7.7 lanes. Here:
+// ray per lane from start to end the lanes of a warp part ways: 14 lanes are busy
+// in a node visit, 5 in a leaf, a leaf runs as long as its largest, and 32 rays take
+// 26.0k warp instructions at 7.7 lanes. Here:
 //  * a leaf is tested by eight lanes at once, whichever lanes own the rays, so
 //    one round of instructions tests four leaves (35 rounds per 32 rays in place
 //    of 20 leaf steps of up to 8 triangles each); the rays' triangle-test
@@ -24,10 +24,10 @@
 // 25.9). Issue slots are then 60% busy and the L1 data pipe is at 73% of its peak
 // (shadow 83%: a divergent 32-byte load per plane and lane, 48 bytes per
 // triangle), with 4.7 warps waiting on loads per issue (5.8); DRAM is at 2%.
-// Before and now, one box: 4,194,304 diffuse rays, 21M triangles, 3.93 ms in sorted
-// order, now 2.15 in batch order; as many shadow rays 3.61 -> 2.05; 1,048,576 camera
-// rays, 82k triangles, width 4, 0.255 -> 0.176; 700,001 diffuse rays, 1.3M
-// triangles, 8-bit nodes 0.744 -> 0.323.
+// One ray per lane against this form, one box: 4,194,304 diffuse rays, 21M triangles,
+// 3.93 ms in sorted order, 2.15 in batch order; as many shadow rays 3.61 / 2.05;
+// 1,048,576 camera rays, 82k triangles, width 4, 0.255 / 0.176; 700,001 diffuse rays,
+// 1.3M triangles, 8-bit nodes 0.744 / 0.323.
 // Slower forms: a second round's triangles fetched ahead (52 bytes spilled,
 // 2.99 ms on the diffuse rays against 2.66), every hit but the nearest pushed and
 // sorted on the stack (2.98), the 1/d and -o/d pairs kept doubled in registers
