@@ -1284,10 +1284,10 @@ BuiltTree build_tree_gpu(const float* tri, int64_t ntri, const BuildParams& p, i
 
     // Rounds are queued in groups without a host round trip (a round with no
     // node left does no work); the host reads the state after each group. A
-    // node splits at most W - 1 times and the depth is capped, which bounds
-    // the rounds.
+    // node splits at most W - 1 times, sets fewer ranges aside (a round each too)
+    // and the depth is capped, which bounds the rounds.
     constexpr int kGroup = 8;
-    const int64_t max_rounds = int64_t(W - 1) * p.max_depth + 1;
+    const int64_t max_rounds = 2 * int64_t(W - 1) * p.max_depth;
     const unsigned ng = grid(cap, 128);
     int64_t queued = 0;
     while (large_root) {
